@@ -61,6 +61,9 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, ui
 
 #define AT_WAIT(bar, ph, site) mbar_wait((bar), (ph), abort_flag, p.status, (site))
 
+// the same by a whole warp, which stays converged
+#define AT_WAIT_ALL(bar, ph, site) __all_sync(0xffffffffu, AT_WAIT(bar, ph, site))
+
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

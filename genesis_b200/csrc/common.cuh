@@ -22,6 +22,17 @@ static inline int smem_opt_in(KernT kern, int bytes, unsigned long long& mask) {
   return 0;
 }
 
+// Number of SMs of the current device (asked for once per device).
+static inline int sm_count() {
+  static int known[64] = {0};
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && known[dev] != 0) return known[dev];
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+  if (dev >= 0 && dev < 64) known[dev] = n;
+  return n;
+}
+
 // dtype codes of the C ABI (mirrored in genesis_b200/ops/native.py)
 enum : int { DT_F32 = 0, DT_F16 = 1, DT_BF16 = 2, DT_F64 = 3, DT_I32 = 4, DT_I64 = 5, DT_U8 = 6, DT_BOOL = 7 };
 

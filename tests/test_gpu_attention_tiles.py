@@ -1,0 +1,76 @@
+"""The attention kernels at the edges of their tiles, work items and routes: 128-row and 128-column tiles, pairs of q
+tiles, groups of query rows that the decoding kernel takes, kv tiles that few queries see, and scores whose maximum keeps
+growing (the accumulator's rescaling).  The oracle is the softmax in float64."""
+import math
+
+import pytest
+import torch
+
+import genesis_b200  # noqa: F401
+from genesis_b200.ops import native as N
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _inputs(B, S, Sk, Hq, Hkv, D, dt, ramp=0.0):
+    g = torch.Generator(device=DEV).manual_seed(B + 3 * S + 5 * Sk + 7 * Hq + D)
+    q = torch.randn(B, S, Hq, D, device=DEV, generator=g)
+    k = torch.randn(B, Sk, Hkv, D, device=DEV, generator=g)
+    v = torch.randn(B, Sk, Hkv, D, device=DEV, generator=g)
+    if ramp:
+        # one shared component of q and k makes the scores climb by `ramp` (natural log) over the keys
+        q[..., 0] = math.sqrt(D)
+        k[..., 0] = torch.linspace(0, ramp, Sk, device=DEV)[None, :, None]
+    return q.to(dt), k.to(dt), v.to(dt)
+
+
+def _oracle(q, k, v, causal, scale):
+    """o, lse and P |v| in float64, laid out as the kernel's."""
+    B, S, Hq, D = q.shape
+    Sk, g = k.shape[1], Hq // k.shape[2]
+    qd, kd, vd = (t.double().transpose(1, 2) for t in (q, k.repeat_interleave(g, 2), v.repeat_interleave(g, 2)))
+    s = qd @ kd.transpose(-1, -2) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(S, Sk, dtype=torch.bool, device=DEV).triu(Sk - S + 1), -math.inf)
+    p = torch.softmax(s, -1)
+    return (p @ vd).transpose(1, 2), torch.logsumexp(s, -1), (p @ vd.abs()).transpose(1, 2)
+
+
+def _check_fwd(q, k, v, causal):
+    D, dt = q.shape[-1], q.dtype
+    scale = D ** -0.5
+    r = N.attention_fwd(q, k, v, causal, scale)
+    assert r is not NotImplemented
+    o, lse = r
+    N.check_status()
+    ref, lref, pv = _oracle(q, k, v, causal, scale)
+    # every probability and the result are rounded once to 16 bits: with p significand bits the relative error of a
+    # rounding is at most 2^-p (8 bits: 2^-8 for bf16, 11 bits: 2^-11 for fp16); fp32 exponents of size x carry
+    # |x| 2^-23, which 2^-16 covers up to |x| = 2^7; fp16 probabilities below 2^-14 are rounded to multiples of 2^-24
+    u = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    tiny = 0.0 if dt == torch.bfloat16 else 2.0 ** -25 * k.shape[1] * float(v.abs().max())
+    bound = (u + 2.0 ** -16) * (pv + ref.abs()) + tiny + 1e-6
+    assert bool(((o.double() - ref).abs() <= bound).all()), float(((o.double() - ref).abs() / bound).max())
+    assert float((lse.double() - lref).abs().max()) <= 2e-5 * max(1.0, float(lref.abs().max()))
+    return o, lse, scale
+
+
+FWD = [
+    # B, S, Sk, Hq, Hkv, D: one tile and its neighbours, one row more than a pair, ragged keys, enough work for pairs
+    (1, 127, 127, 2, 1, 64), (1, 129, 129, 9, 3, 64), (1, 255, 300, 2, 2, 128), (2, 257, 257, 4, 2, 128),
+    (1, 385, 1000, 14, 2, 64), (3, 640, 640, 40, 8, 64), (2, 513, 513, 80, 16, 128), (40, 130, 131, 4, 4, 64),
+]
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("case", FWD)
+@pytest.mark.parametrize("causal", [True, False])
+def test_forward_at_tile_edges(case, dt, causal):
+    _check_fwd(*_inputs(*case, dt), causal)
+
+
+@pytest.mark.parametrize("shape", [(1, 700, 700, 2, 1, 64), (1, 300, 900, 2, 2, 128)])
+@pytest.mark.parametrize("ramp", [60.0, -60.0])
+def test_forward_with_growing_scores(shape, ramp):
+    _check_fwd(*_inputs(*shape, torch.bfloat16, ramp=ramp), True)
