@@ -1,22 +1,36 @@
-// Flash-attention backward for sm_100a (tcgen05 / TMEM / TMA): dQ kernel, dK/dV kernel, delta pre-pass.
+// Flash-attention backward for sm_100a (tcgen05 / TMEM / TMA): row statistics, dQ kernel, dK/dV kernel.
 //
-// Both kernels work on 128 x 64 score tiles: 128 row threads (one TMEM lane each) by 64 columns, which
-// keeps S and dP (64 + 64 fp32 registers per thread) in registers after ONE tensor-memory round trip, so
-// the TMEM tile is handed back at once and the next tile's QK^T / dO V^T run while the current tile's
-// exponentials are computed.  Operand tiles arrive through a TMA ring (three stages in dQ, two in dK/dV).
-//   dQ    : CTA = (q tile of 128 rows, head); loop over kv tiles of 64:
+// Both kernels work on 128 x 128 score tiles with eight arithmetic warps: two warpgroups share a tile by columns (64
+// each), every thread owns one row of its half (one TMEM lane).  A TMA warp feeds a ring of operand tiles, an MMA warp
+// issues.  P and dS never pass through shared memory: they are written as 16-bit pairs into tensor memory, as the A
+// operand of the GEMM that consumes them.
+//   dQ    : CTA = (q tile of 128 rows, head); loop over kv tiles:
 //           S = Q K^T, dP = dO V^T, dS = P o (dP - delta) * scale, dQ += dS K          (K tile reused MN-major)
-//   dK/dV : CTA = (kv tile of 128 rows, query head); loop over q tiles of 64:
+//           S and dP of tile j + 1 are issued as soon as those of tile j are in registers, ahead of dQ(j).
+//   dK/dV : CTA = (kv tile of 128 rows, some query heads of its group); loop over those heads and their q tiles:
 //           S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q                     (dO, Q tiles reused MN-major)
-// With D = 64 a CTA needs 256 TMEM columns and at most 100.1 KB of shared memory: two CTAs share an SM.
+//           P^T replaces S^T and dS^T replaces dP^T in place, so at D = 128 the four tiles fill the 512 columns; the two
+//           halves of an iteration alternate: while the warps form dS^T(i) the tensor cores run dV(i) and S^T(i + 1),
+//           while they exponentiate S^T(i + 1) the tensor cores run dK(i) and dP^T(i + 1).
+// What bounds them: 3 + 4 GEMMs of 128 x 128 x D per score tile (each 512 clocks at D = 128, 256 at D = 64, at the nominal
+// rate) against one exponential per score in each kernel (1024 clocks): the tensor pipe at D = 128, the exponentials at D = 64.
+// Measured against the kernels they replace (128 x 64 tiles, four arithmetic warps, one dK/dV CTA per query head with fp32
+// atomics for every group), whole backward pass, bf16 causal, us: 8 x 2048, 14 / 2 heads of 64: 538 -> 324; 4 x 4096,
+// 12 / 2 of 128: 1437 -> 680; 8 x 1024, 16 / 4 of 128: 436 -> 180; 1 x 1003, 14 / 2 of 64: 80 -> 56.
 // Reference counterpart: genesis/nn/attention.py:162-406 (Triton, 32 x 32 tiles, Hq == Hkv only).
 #include "attention_common.cuh"
 
 namespace gb {
 
-constexpr int BW_C = 64;    // columns of a backward score tile
-constexpr int BW_ST = 3;    // stages of the ring of streamed operand tiles in the dQ kernel
-constexpr int KV_ST = 2;    // ... and in the dK/dV kernel, which spends the shared memory on per-warp statistics instead
+constexpr int BW_THREADS = 320;     // 2 x 4 arithmetic warps, TMA warp, MMA warp
+
+template <int D> struct BwdCfg {
+  static constexpr int TILE = AT_BM * D * 2;                    // one [128 x D] 16-bit tile
+  static constexpr int ST = D == 64 ? 3 : 2;                    // stages of the operand ring (two tiles each)
+  static constexpr int STATS = 2 * AT_BM * 4;                   // -lse (log2 domain) and -delta of a q tile
+  static constexpr int SMEM_DQ = 2 * TILE + ST * 2 * TILE + 256;
+  static constexpr int SMEM_KV = 2 * TILE + ST * (2 * TILE + STATS) + 256;
+};
 
 __device__ __forceinline__ void store_out_row(uint16_t* dst, uint32_t tsrc, int ncols, bool valid, int dt,
                                               float mul = 1.f) {
@@ -42,14 +56,13 @@ __device__ __forceinline__ void store_out_row(uint16_t* dst, uint32_t tsrc, int 
 // =====================================================================================================
 // dQ
 // =====================================================================================================
-template <int D, int NCTA>
-__global__ void __maxnreg__(NCTA == 2 ? 168 : 255)
+template <int D, bool BF16>
+__global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                    const __grid_constant__ CUtensorMap tmv, const __grid_constant__ CUtensorMap tmdo,
                    const AttnParams p) {
-  constexpr int QT = AT_BM * D * 2;          // [128 x D] tile
-  constexpr int KT = BW_C * D * 2;           // [64 x D] tile
-  constexpr uint32_t TCOLS = (D == 64) ? 256 : 512;   // 64 (S) + 64 (dP) + D (dQ) + 32 (dS as 16-bit pairs)
+  using C = BwdCfg<D>;
+  constexpr int TILE = C::TILE, ST = C::ST;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (status_poisoned(p.status)) return;
   if ((reinterpret_cast<uintptr_t>(smem_raw) & 1023) != 0) {
@@ -57,173 +70,195 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
     return;
   }
   uint8_t* sQ = smem_raw;
-  uint8_t* sdO = sQ + QT;
-  uint8_t* sK = sdO + QT;            // BW_ST stages
-  uint8_t* sV = sK + BW_ST * KT;     // BW_ST stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + BW_ST * KT);
+  uint8_t* sdO = sQ + TILE;
+  uint8_t* sKV = sdO + TILE;         // ST stages of (K, V)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + ST * 2 * TILE);
   uint64_t* qdo_full = bars;
-  uint64_t* kv_full = bars + 1;      // [BW_ST]
-  uint64_t* sdp_full = bars + 4;
-  uint64_t* sdp_free = bars + 5;
-  uint64_t* ds_ready = bars + 6;
-  uint64_t* acc_done = bars + 7;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* s_full = bars + 1;
+  uint64_t* dp_full = bars + 2;
+  uint64_t* s_free = bars + 3;
+  uint64_t* dp_free = bars + 4;
+  uint64_t* ds_ready = bars + 5;
+  uint64_t* acc_done = bars + 6;
+  uint64_t* kv_full = bars + 7;      // [ST]
+  uint64_t* kv_empty = bars + 7 + ST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7 + 2 * ST);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int bh = p.B * p.Hq, nq = (p.S + AT_BM - 1) / AT_BM;
+  const int qt = nq - 1 - (int)blockIdx.x / bh;           // longest (last) rows first
+  const int h = (int)blockIdx.x % bh % p.Hq, b = (int)blockIdx.x % bh / p.Hq;
   const int kvh = h / (p.Hq / p.Hkv);
   const int m0 = qt * AT_BM;
   const int off = p.Sk - p.S;
-  int n_kv = (p.Sk + BW_C - 1) / BW_C;
+  int n_kv = (p.Sk + AT_BN - 1) / AT_BN;
   if (p.causal) {
-    const int lim = (m0 + AT_BM + off + BW_C - 1) / BW_C;
+    const int lim = (m0 + AT_BM + off + AT_BN - 1) / AT_BN;
     n_kv = lim < n_kv ? lim : n_kv;
   }
   if (n_kv < 1) n_kv = 1;
 
   if (threadIdx.x == 0) {
-    mbar_init(qdo_full, 1); mbar_init(sdp_full, 1);
-    for (int i = 0; i < BW_ST; ++i) mbar_init(&kv_full[i], 1);
-    mbar_init(sdp_free, 128); mbar_init(ds_ready, 128); mbar_init(acc_done, 1);
+    mbar_init(qdo_full, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1); mbar_init(acc_done, 1);
+    mbar_init(s_free, 256); mbar_init(dp_free, 256); mbar_init(ds_ready, 256);
+    for (int i = 0; i < ST; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4) { tmem_alloc(tmem_slot, TCOLS); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + BW_C, tdQ = tmem + 2 * BW_C, tdS = tmem + 2 * BW_C + D;
+  const uint32_t tS = tmem, tdP = tmem + 128, tdS = tmem + 256, tdQ = tmem + 320;   // 128 + 128 + 64 + D columns
 
-  if (warp == 4) {
-    if (lane == 0) {   // ---------------- TMA + MMA ----------------
-      const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-      const uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, BW_C);
-      const uint32_t idesc_dq = make_idesc(fmt, 0, 1, AT_BM, D);
-      const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO);
-      auto load_kv = [&](int j) {
-        const int st = j % BW_ST;
-        mbar_expect_tx(&kv_full[st], 2 * KT);
-        load_tile<D>(sK + st * KT, &tmk, &kv_full[st], kvh, j * BW_C, b, BW_C);
-        load_tile<D>(sV + st * KT, &tmv, &kv_full[st], kvh, j * BW_C, b, BW_C);
-      };
-      auto issue_s = [&](int j) -> bool {
-        const int st = j % BW_ST;
-        if (!AT_WAIT(&kv_full[st], (j / BW_ST) & 1, 42)) return false;
-        if (j > 0 && !AT_WAIT(sdp_free, (j - 1) & 1, 44)) return false;
-        tc_fence_after_sync();
-        const uint32_t aK = smem_u32(sK + st * KT), aV = smem_u32(sV + st * KT);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          umma_f16(tS, desc_kmajor(aQ, kk, AT_BM), desc_kmajor(aK, kk, BW_C), idesc_s, kk > 0);
-          umma_f16(tdP, desc_kmajor(adO, kk, AT_BM), desc_kmajor(aV, kk, BW_C), idesc_s, kk > 0);
-        }
-        umma_commit(sdp_full);
-        return true;
-      };
-      mbar_expect_tx(qdo_full, 2 * QT);
+  if (warp == 8) {
+    if (lane == 0) {   // ---------------- TMA ----------------
+      mbar_expect_tx(qdo_full, 2 * TILE);
       load_tile<D>(sQ, &tmq, qdo_full, h, m0, b, AT_BM);
       load_tile<D>(sdO, &tmdo, qdo_full, h, m0, b, AT_BM);
-      for (int j = 0; j < BW_ST && j < n_kv; ++j) load_kv(j);
-      bool ok = AT_WAIT(qdo_full, 0, 41) && issue_s(0);
-      for (int j = 0; ok && j < n_kv; ++j) {
-        if (j + 1 < n_kv && !issue_s(j + 1)) break;
-        if (!AT_WAIT(ds_ready, j & 1, 43)) break;
-        tc_fence_after_sync();
-        const uint32_t aK = smem_u32(sK + (j % BW_ST) * KT);
-#pragma unroll
-        for (int kk = 0; kk < BW_C / 16; ++kk)
-          umma_f16_ts(tdQ, tdS + kk * 8, desc_mnmajor(aK, kk, BW_C), idesc_dq, (j > 0 || kk > 0));
-        umma_commit(acc_done);
-        // tile j - 1 is retired (the row threads waited for it before they signalled ds_ready(j)): refill
-        // its stage with tile j - 1 + BW_ST, a full iteration before anything needs it
-        // (no wait on acc_done here: its phase j - 1 is known complete, and a parity wait issued after the
-        // commit above could alias phase j + 1)
-        if (j >= 1 && j - 1 + BW_ST < n_kv) load_kv(j - 1 + BW_ST);
+      for (int j = 0; j < n_kv; ++j) {
+        const int st = j % ST;
+        if (!AT_WAIT(&kv_empty[st], ((j / ST) & 1) ^ 1, 40)) break;
+        mbar_expect_tx(&kv_full[st], 2 * TILE);
+        load_tile<D>(sKV + st * 2 * TILE, &tmk, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
+        load_tile<D>(sKV + st * 2 * TILE + TILE, &tmv, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
       }
     }
+  } else if (warp == 9) {
+    // ---------------- MMA: the warp stays converged, one elected lane issues ----------------
+    constexpr uint32_t fmt = BF16 ? 1u : 0u;
+    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, AT_BN);
+    constexpr uint32_t idesc_dq = make_idesc(fmt, 0, 1, AT_BM, D);
+    const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO), aKV = smem_u32(sKV);
+    auto score = [&](uint32_t d, uint32_t a, uint32_t bb, uint64_t* done) {
+      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, AT_BN);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t o = (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2;
+          umma_f16(d, da + o, db + o, idesc_s, kk > 0);
+        }
+        umma_commit(done);
+      }
+      __syncwarp();
+    };
+    bool ok = AT_WAIT_ALL(qdo_full, 0, 41) && AT_WAIT_ALL(&kv_full[0], 0, 42);
+    if (ok) {
+      tc_fence_after_sync();
+      score(tS, aQ, aKV, s_full);
+      score(tdP, adO, aKV + TILE, dp_full);
+    }
+    for (int j = 0; ok && j < n_kv; ++j) {
+      if (j + 1 < n_kv) {
+        const int st = (j + 1) % ST;
+        if (!(ok = AT_WAIT_ALL(&kv_full[st], ((j + 1) / ST) & 1, 43) && AT_WAIT_ALL(s_free, j & 1, 44))) break;
+        tc_fence_after_sync();
+        score(tS, aQ, aKV + st * 2 * TILE, s_full);
+        if (!(ok = AT_WAIT_ALL(dp_free, j & 1, 45))) break;
+        tc_fence_after_sync();
+        score(tdP, adO, aKV + st * 2 * TILE + TILE, dp_full);
+      }
+      if (!(ok = AT_WAIT_ALL(ds_ready, j & 1, 46))) break;
+      tc_fence_after_sync();
+      const uint64_t dk = desc_mnmajor(aKV + (j % ST) * 2 * TILE, 0, AT_BN);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < AT_BN / 16; ++kk)
+          umma_f16_ts(tdQ, tdS + kk * 8, dk + kk * (2048 / 16), idesc_dq, j > 0 || kk > 0);
+        umma_commit(acc_done);
+        umma_commit(&kv_empty[j % ST]);
+      }
+      __syncwarp();
+    }
   } else {
-    const int t = threadIdx.x;
-    const int row = m0 + t;
-    const uint32_t lane_base = ((uint32_t)(warp * 32)) << 16;
+    const int half = warp >> 2;                          // columns half * 64 .. + 63 of every score tile
+    const int row = m0 + (threadIdx.x & 127);
+    const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
     const float sl2 = p.scale * LOG2E;
-    const size_t stat = ((size_t)b * p.Hq + h) * p.S + row;
-    const float lse2 = row < p.S ? p.lse_in[stat] * LOG2E : 0.f;
-    const float dl = row < p.S ? p.delta[stat] : 0.f;
+    const float2 sl2v = make_float2(sl2, sl2);
+    const float* stat = p.stats + ((size_t)b * p.Hq + h) * p.Spad + row;
+    const float nl = stat[0], nd = stat[(size_t)p.B * p.Hq * p.Spad];
+    const float2 nlv = make_float2(nl, nl), ndv = make_float2(nd, nd);
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!__all_sync(0xffffffffu, AT_WAIT(sdp_full, j & 1, 50))) { ok = false; break; }
+      if (!(ok = AT_WAIT_ALL(s_full, j & 1, 50))) break;
       tc_fence_after_sync();
-      uint32_t rs[2][32], rp[2][32];
-      tmem_ld_32x32b_x32(tS + lane_base, rs[0]);
-      tmem_ld_32x32b_x32(tS + lane_base + 32, rs[1]);
-      tmem_ld_32x32b_x32(tdP + lane_base, rp[0]);
-      tmem_ld_32x32b_x32(tdP + lane_base + 32, rp[1]);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      mbar_arrive(sdp_free);
-      const int col0 = j * BW_C;
-      const bool need_mask = (col0 + BW_C > p.Sk) || (p.causal && (col0 + BW_C - 1 > m0 + off)) || (m0 + AT_BM > p.S);
-      if (need_mask) {
-        // masked scores become -inf (probability 0) in a pass of their own: the main loop stays branch-free
-        int lim = p.causal ? row + off : p.Sk - 1;            // last visible column of this row
-        lim = lim < p.Sk - 1 ? lim : p.Sk - 1;
-        if (row >= p.S) lim = -1;
-        lim -= col0;
+      float pr[64];
+      {
+        uint32_t s[2][32];
+        tmem_ld_32x32b_x32(tS + lane_base + half * 64, s[0]);
+        tmem_ld_32x32b_x32(tS + lane_base + half * 64 + 32, s[1]);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        mbar_arrive(s_free);
+        const int col0 = j * AT_BN;
+        if ((col0 + AT_BN > p.Sk) || (p.causal && (col0 + AT_BN - 1 > m0 + off)) || (m0 + AT_BM > p.S)) {
+          // masked scores become -inf (probability 0) in a pass of their own: the main loop stays branch-free
+          int lim = p.causal ? row + off : p.Sk - 1;            // last visible column of this row
+          lim = lim < p.Sk - 1 ? lim : p.Sk - 1;
+          if (row >= p.S) lim = -1;
+          lim -= col0 + half * 64;
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) rs[c][i] = (c * 32 + i <= lim) ? rs[c][i] : 0xff800000u;
-      }
-      // dS = P o (dP - delta) as 16-bit pairs (the softmax scale is applied once, to dQ at the end)
-      uint32_t dsp[32];
+            for (int i = 0; i < 32; ++i) s[c][i] = (c * 32 + i <= lim) ? s[c][i] : 0xff800000u;
+        }
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(rs[c][i]), sl2, -lse2));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(rs[c][i + 1]), sl2, -lse2));
-          const float d0 = p0 * (__uint_as_float(rp[c][i]) - dl);
-          const float d1 = p1 * (__uint_as_float(rp[c][i + 1]) - dl);
-          dsp[c * 16 + i / 2] = p.is_bf16 ? pack2c<true>(d0, d1) : pack2c<false>(d0, d1);
+        for (int i = 0; i < 64; i += 2) {
+          const float2 x = fma2(make_float2(__uint_as_float(s[i >> 5][i & 31]), __uint_as_float(s[i >> 5][(i & 31) + 1])),
+                                sl2v, nlv);
+          pr[i] = fast_exp2(x.x);
+          pr[i + 1] = fast_exp2(x.y);
         }
       }
-      // dS lives in tensor memory (A operand of the dQ MMA), single-buffered: the previous iteration's MMA has
-      // to be done reading it
-      if (j > 0 && !__all_sync(0xffffffffu, AT_WAIT(acc_done, (j - 1) & 1, 51))) { ok = false; break; }
+      if (!(ok = AT_WAIT_ALL(dp_full, j & 1, 51))) break;
       tc_fence_after_sync();
-      tmem_st_32x32b_x32(tdS + lane_base, dsp);
+      uint32_t dp[2][32], ds[32];
+      tmem_ld_32x32b_x32(tdP + lane_base + half * 64, dp[0]);
+      tmem_ld_32x32b_x32(tdP + lane_base + half * 64 + 32, dp[1]);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      mbar_arrive(dp_free);
+      // dS = P o (dP - delta) as 16-bit pairs (the softmax scale is applied once, to dQ at the end)
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        const float2 d = mul2(make_float2(pr[i], pr[i + 1]),
+                              add2(make_float2(__uint_as_float(dp[i >> 5][i & 31]), __uint_as_float(dp[i >> 5][(i & 31) + 1])), ndv));
+        ds[i / 2] = pack2c<BF16>(d.x, d.y);
+      }
+      // dS is single-buffered: the previous tile's dQ MMA has to be done reading it
+      if (j > 0 && !(ok = AT_WAIT_ALL(acc_done, (j - 1) & 1, 52))) break;
+      tc_fence_after_sync();
+      tmem_st_32x32b_x32(tdS + lane_base + half * 32, ds);
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(ds_ready);
     }
-    if (ok && __all_sync(0xffffffffu, AT_WAIT(acc_done, (n_kv - 1) & 1, 52))) {
+    if (ok && AT_WAIT_ALL(acc_done, (n_kv - 1) & 1, 53)) {
       tc_fence_after_sync();
-      uint16_t* drow = reinterpret_cast<uint16_t*>(p.dq) + (((size_t)b * p.S + row) * p.Hq + h) * D;
-      store_out_row(drow, tdQ + lane_base, D, row < p.S, p.is_bf16 ? DT_BF16 : DT_F16, p.scale);
+      uint16_t* drow = reinterpret_cast<uint16_t*>(p.dq) + (((size_t)b * p.S + row) * p.Hq + h) * D + half * (D / 2);
+      store_out_row(drow, tdQ + lane_base + half * (D / 2), D / 2, row < p.S, BF16 ? DT_BF16 : DT_F16, p.scale);
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 4) { tc_fence_after_sync(); tmem_dealloc(tmem, TCOLS); }
+  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
 }
 
 // =====================================================================================================
-// dK / dV.  One CTA per (kv tile of 128 rows, QUERY head, batch): with grouped-query attention the heads of
-// a group add their parts into an fp32 workspace (vector atomics), which keeps the grid large and the
-// causal triangle balanced; with Hq == Hkv the CTA owns its output rows and stores them directly.
+// dK / dV.  One CTA per (kv tile of 128 rows, `1 / splits` of the query heads of a KV head's group, batch).  With
+// splits == 1 the CTA owns its output rows and stores them; otherwise (too few kv tiles to fill the GPU with whole
+// groups) the parts are added into an fp32 workspace with vector atomics.
 // =====================================================================================================
-template <int D, int NCTA>
-__global__ void __maxnreg__(NCTA == 2 ? 168 : 255)
+template <int D, bool BF16>
+__global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                      const __grid_constant__ CUtensorMap tmv, const __grid_constant__ CUtensorMap tmdo,
-                     const AttnParams p, float* __restrict__ ws) {
-  constexpr int KT = AT_BM * D * 2;          // [128 x D] K / V tile
-  constexpr int QT = BW_C * D * 2;           // [64 x D] Q / dO tile
-  constexpr int PB = AT_BM * BW_C * 2;       // [128 x 64] 16-bit tile
-  constexpr uint32_t TCOLS = (D == 64) ? 256 : 512;   // 64 (S^T) + 64 (dP^T) + D (dV) + D (dK)
+                     const AttnParams p, float* __restrict__ ws, const int splits) {
+  using C = BwdCfg<D>;
+  constexpr int TILE = C::TILE, ST = C::ST, STAGE = 2 * TILE;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (status_poisoned(p.status)) return;
   if ((reinterpret_cast<uintptr_t>(smem_raw) & 1023) != 0) {
@@ -231,213 +266,219 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
     return;
   }
   uint8_t* sK = smem_raw;
-  uint8_t* sV = sK + KT;
-  uint8_t* sQ = sV + KT;             // KV_ST stages
-  uint8_t* sdO = sQ + KV_ST * QT;    // KV_ST stages
-  uint8_t* sPT = sdO + KV_ST * QT;
-  uint8_t* sdST = sPT + PB;
-  float* lse_s = reinterpret_cast<float*>(sdST + PB);     // [4 warps][2][64] log2-domain row statistics, a copy per warp
-  float* dl_s = lse_s + 8 * BW_C;                          // [4 warps][2][64] delta
-  uint64_t* bars = reinterpret_cast<uint64_t*>(dl_s + 8 * BW_C);
+  uint8_t* sV = sK + TILE;
+  uint8_t* sQ = sV + TILE;           // ST stages of (Q, dO)
+  uint8_t* sStat = sQ + ST * STAGE;  // ST stages of 128 x (-lse), 128 x (-delta)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + ST * C::STATS);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;     // [KV_ST]
-  uint64_t* sdp_full = bars + 4;
-  uint64_t* sdp_free = bars + 5;
-  uint64_t* ds_ready = bars + 6;
-  uint64_t* acc_done = bars + 7;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* s_full = bars + 1;
+  uint64_t* dp_full = bars + 2;
+  uint64_t* p_ready = bars + 3;
+  uint64_t* ds_ready = bars + 4;
+  uint64_t* acc_done = bars + 5;
+  uint64_t* q_full = bars + 6;       // [ST]
+  uint64_t* q_empty = bars + 6 + ST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 2 * ST);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int group = p.Hq / p.Hkv;
-  const int kvh = h / group;
-  const int n0 = blockIdx.x * AT_BM;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int group = p.Hq / p.Hkv, parts = p.Hkv * splits;
+  const int r = (int)blockIdx.x % (parts * p.B), hs = r % parts, b = r / parts;
+  const int n0 = (int)blockIdx.x / (parts * p.B) * AT_BM;     // first kv tiles first: they see the most queries
+  const int kvh = hs / splits, part = hs % splits;
+  const int h0 = kvh * group + part * group / splits, h1 = kvh * group + (part + 1) * group / splits;
   const int off = p.Sk - p.S;
-  const int nq = (p.S + BW_C - 1) / BW_C;
+  const int nq = (p.S + AT_BM - 1) / AT_BM;
   int i_start = 0;
-  if (p.causal) { const int first = n0 - off; i_start = first > 0 ? first / BW_C : 0; }
-  const int n_it = nq > i_start ? nq - i_start : 0;
+  if (p.causal) { const int first = n0 - off; i_start = first > 0 ? first / AT_BM : 0; }
+  const int nqv = nq > i_start ? nq - i_start : 0;
+  const int n_it = nqv * (h1 - h0);
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1); mbar_init(sdp_full, 1);
-    for (int i = 0; i < KV_ST; ++i) mbar_init(&qdo_full[i], 1);
-    mbar_init(sdp_free, 128); mbar_init(ds_ready, 128); mbar_init(acc_done, 1);
+    mbar_init(kv_full, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1); mbar_init(acc_done, 1);
+    mbar_init(p_ready, 256); mbar_init(ds_ready, 256);
+    for (int i = 0; i < ST; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4) { tmem_alloc(tmem_slot, TCOLS); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tST = tmem, tdPT = tmem + BW_C, tdV = tmem + 2 * BW_C, tdK = tmem + 2 * BW_C + D;
+  const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 256 + D;
 
-  if (warp == 4) {
-    if (lane == 0 && n_it > 0) {   // ---------------- TMA + MMA ----------------
-      const uint32_t fmt = p.is_bf16 ? 1u : 0u;
-      const uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, BW_C);
-      const uint32_t idesc_acc = make_idesc(fmt, 0, 1, AT_BM, D);
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aPT = smem_u32(sPT), adST = smem_u32(sdST);
-      auto load_q = [&](int it) {
-        const int st = it % KV_ST;
-        const int q0 = (i_start + it) * BW_C;
-        mbar_expect_tx(&qdo_full[st], 2 * QT);
-        load_tile<D>(sQ + st * QT, &tmq, &qdo_full[st], h, q0, b, BW_C);
-        load_tile<D>(sdO + st * QT, &tmdo, &qdo_full[st], h, q0, b, BW_C);
-      };
-      auto issue_s = [&](int it) -> bool {
-        const int st = it % KV_ST;
-        if (!AT_WAIT(&qdo_full[st], (it / KV_ST) & 1, 62)) return false;
-        if (it > 0 && !AT_WAIT(sdp_free, (it - 1) & 1, 64)) return false;
-        tc_fence_after_sync();
-        const uint32_t aQ = smem_u32(sQ + st * QT), adO = smem_u32(sdO + st * QT);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          umma_f16(tST, desc_kmajor(aK, kk, AT_BM), desc_kmajor(aQ, kk, BW_C), idesc_s, kk > 0);
-          umma_f16(tdPT, desc_kmajor(aV, kk, AT_BM), desc_kmajor(adO, kk, BW_C), idesc_s, kk > 0);
-        }
-        umma_commit(sdp_full);
-        return true;
-      };
-      mbar_expect_tx(kv_full, 2 * KT);
+  if (warp == 8) {
+    if (lane == 0 && n_it > 0) {   // ---------------- TMA ----------------
+      mbar_expect_tx(kv_full, 2 * TILE);
       load_tile<D>(sK, &tmk, kv_full, kvh, n0, b, AT_BM);
       load_tile<D>(sV, &tmv, kv_full, kvh, n0, b, AT_BM);
-      for (int it = 0; it < KV_ST && it < n_it; ++it) load_q(it);
-      bool ok = AT_WAIT(kv_full, 0, 61) && issue_s(0);
-      for (int it = 0; ok && it < n_it; ++it) {
-        if (it + 1 < n_it && !issue_s(it + 1)) break;
-        if (!AT_WAIT(ds_ready, it & 1, 63)) break;
-        tc_fence_after_sync();
-        const uint32_t aQ = smem_u32(sQ + (it % KV_ST) * QT), adO = smem_u32(sdO + (it % KV_ST) * QT);
-#pragma unroll
-        for (int kk = 0; kk < BW_C / 16; ++kk) {
-          umma_f16(tdV, desc_kmajor(aPT, kk, AT_BM), desc_mnmajor(adO, kk, BW_C), idesc_acc, (it > 0 || kk > 0));
-          umma_f16(tdK, desc_kmajor(adST, kk, AT_BM), desc_mnmajor(aQ, kk, BW_C), idesc_acc, (it > 0 || kk > 0));
-        }
-        umma_commit(acc_done);
-        // two stages: the stage of tile `it` is free once the MMAs just committed are done (a wait on the phase
-        // that was committed last cannot alias)
-        if (it + KV_ST < n_it) {
-          if (!AT_WAIT(acc_done, it & 1, 60)) break;
-          load_q(it + KV_ST);
-        }
+      const size_t half = (size_t)p.B * p.Hq * p.Spad;
+      int h = h0, qt = i_start;
+      for (int it = 0; it < n_it; ++it) {
+        const int st = it % ST;
+        if (!AT_WAIT(&q_empty[st], ((it / ST) & 1) ^ 1, 60)) break;
+        mbar_expect_tx(&q_full[st], STAGE + C::STATS);
+        load_tile<D>(sQ + st * STAGE, &tmq, &q_full[st], h, qt * AT_BM, b, AT_BM);
+        load_tile<D>(sQ + st * STAGE + TILE, &tmdo, &q_full[st], h, qt * AT_BM, b, AT_BM);
+        const float* src = p.stats + ((size_t)b * p.Hq + h) * p.Spad + (size_t)qt * AT_BM;
+        bulk_load(sStat + st * C::STATS, src, AT_BM * 4, &q_full[st]);
+        bulk_load(sStat + st * C::STATS + AT_BM * 4, src + half, AT_BM * 4, &q_full[st]);
+        if (++qt == nq) { qt = i_start; ++h; }
       }
+    }
+  } else if (warp == 9) {
+    // ---------------- MMA: the warp stays converged, one elected lane issues ----------------
+    constexpr uint32_t fmt = BF16 ? 1u : 0u;
+    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, AT_BN);
+    constexpr uint32_t idesc_acc = make_idesc(fmt, 0, 1, AT_BM, D);
+    const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ);
+    auto score = [&](uint32_t d, uint32_t a, uint32_t bb, uint64_t* done) {
+      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, AT_BN);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t o = (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2;
+          umma_f16(d, da + o, db + o, idesc_s, kk > 0);
+        }
+        umma_commit(done);
+      }
+      __syncwarp();
+    };
+    // acc (+)= A B: A = 16-bit pairs in tensor memory, columns 0..31 for k < 64 and 64..95 behind them (each
+    // warpgroup packs into the columns it read), B = an operand tile as MN-major
+    auto accumulate = [&](uint32_t d, uint32_t a, uint32_t tile, bool first) {
+      const uint64_t db = desc_mnmajor(tile, 0, AT_BN);
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < AT_BN / 16; ++kk)
+          umma_f16_ts(d, a + (kk >> 2) * 64 + (kk & 3) * 8, db + kk * (2048 / 16), idesc_acc, !first || kk > 0);
+      }
+      __syncwarp();
+    };
+    bool ok = n_it > 0 && AT_WAIT_ALL(kv_full, 0, 61) && AT_WAIT_ALL(&q_full[0], 0, 62);
+    if (ok) {
+      tc_fence_after_sync();
+      score(tS, aK, aQ, s_full);
+      score(tdP, aV, aQ + TILE, dp_full);
+    }
+    for (int it = 0; ok && it < n_it; ++it) {
+      const uint32_t cur = aQ + (it % ST) * STAGE, nxt = aQ + ((it + 1) % ST) * STAGE;
+      const bool more = it + 1 < n_it;
+      if (!(ok = AT_WAIT_ALL(p_ready, it & 1, 63))) break;
+      tc_fence_after_sync();
+      accumulate(tdV, tS, cur + TILE, it == 0);
+      if (more) {
+        if (!(ok = AT_WAIT_ALL(&q_full[(it + 1) % ST], ((it + 1) / ST) & 1, 64))) break;
+        tc_fence_after_sync();
+        score(tS, aK, nxt, s_full);
+      }
+      if (!(ok = AT_WAIT_ALL(ds_ready, it & 1, 65))) break;
+      tc_fence_after_sync();
+      accumulate(tdK, tdP, cur, it == 0);
+      if (elect_one()) umma_commit(more ? &q_empty[it % ST] : acc_done);
+      __syncwarp();
+      if (more) score(tdP, aV, nxt + TILE, dp_full);
     }
   } else {
-    const int t = threadIdx.x;
-    const int kvrow = n0 + t;
-    const uint32_t lane_base = ((uint32_t)(warp * 32)) << 16;
+    const int half = warp >> 2;                          // columns half * 64 .. + 63 of every score tile
+    const int kvrow = n0 + (threadIdx.x & 127);
+    const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
+    const uint32_t tSh = tS + lane_base + half * 64, tdPh = tdP + lane_base + half * 64;
     const float sl2 = p.scale * LOG2E;
-    const size_t stat0 = ((size_t)b * p.Hq + h) * p.S;
+    const float2 sl2v = make_float2(sl2, sl2);
     bool ok = true;
-    // Per-column statistics (log2-domain LSE, delta) of a q tile: each warp keeps its own copy in shared memory,
-    // double-buffered; a lane fetches two columns of the NEXT tile into registers at the top of an iteration and
-    // parks them in the other buffer at its end, so the global latency hides behind the tile's arithmetic.
-    auto fetch_stats = [&](int it, float (&v)[4]) {
-      const int q0n = (i_start + it) * BW_C;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int qr = q0n + lane + u * 32;
-        v[u] = qr < p.S ? p.lse_in[stat0 + qr] * LOG2E : 0.f;
-        v[2 + u] = qr < p.S ? p.delta[stat0 + qr] : 0.f;
-      }
-    };
-    auto park_stats = [&](int it, const float (&v)[4]) {
-      float* lb = lse_s + (warp * 2 + (it & 1)) * BW_C;
-      float* db = dl_s + (warp * 2 + (it & 1)) * BW_C;
-      lb[lane] = v[0]; lb[lane + 32] = v[1]; db[lane] = v[2]; db[lane + 32] = v[3];
-    };
-    if (n_it > 0) {
-      float v0[4];
-      fetch_stats(0, v0);
-      park_stats(0, v0);
-      __syncwarp();
-    }
+    int qt = i_start;
     for (int it = 0; it < n_it; ++it) {
-      const int q0 = (i_start + it) * BW_C;
-      float nxt[4] = {0.f, 0.f, 0.f, 0.f};
-      if (it + 1 < n_it) fetch_stats(it + 1, nxt);
-      const float* lse_b = lse_s + (warp * 2 + (it & 1)) * BW_C;
-      const float* dl_b = dl_s + (warp * 2 + (it & 1)) * BW_C;
-      if (!__all_sync(0xffffffffu, AT_WAIT(sdp_full, it & 1, 70))) { ok = false; break; }
+      const int q0 = qt * AT_BM + half * 64;
+      if (++qt == nq) qt = i_start;
+      const int st = it % ST;
+      const float4* nl = reinterpret_cast<const float4*>(sStat + st * C::STATS + half * 256);
+      const float4* nd = reinterpret_cast<const float4*>(sStat + st * C::STATS + AT_BM * 4 + half * 256);
+      // (the statistics are this stage's own: seen through the barrier that their copy completed on)
+      if (!(ok = AT_WAIT_ALL(&q_full[st], (it / ST) & 1, 70) && AT_WAIT_ALL(s_full, it & 1, 71))) break;
       tc_fence_after_sync();
-      const bool need_mask = (q0 + BW_C > p.S) || (n0 + AT_BM > p.Sk) || (p.causal && (n0 + AT_BM - 1 > q0 + off));
-      // this kv row is visible to query columns first..last of the tile
-      const int first = p.causal ? kvrow - off - q0 : 0;
-      const int last = kvrow < p.Sk ? p.S - 1 - q0 : -1;
-      // two half tiles of 32 columns, each read from tensor memory just before its use: 64 live accumulator
-      // registers instead of 128 keep the kernel at two CTAs per SM
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t rs[32], rp[32];
-        tmem_ld_32x32b_x32(tST + lane_base + c * 32, rs);
-        tmem_ld_32x32b_x32(tdPT + lane_base + c * 32, rp);
+      float pr[64];
+      {
+        uint32_t s[2][32], pk[32];
+        tmem_ld_32x32b_x32(tSh, s[0]);
+        tmem_ld_32x32b_x32(tSh + 32, s[1]);
         tmem_ld_wait();
-        if (c == 1) { tc_fence_before_sync(); mbar_arrive(sdp_free); }
-        if (need_mask) {
+        if ((q0 + 64 > p.S) || (n0 + AT_BM > p.Sk) || (p.causal && (n0 + AT_BM - 1 > q0 + off))) {
+          // this kv row is visible to query columns first..last of the half tile
+          const int first = p.causal ? kvrow - off - q0 : 0;
+          const int last = kvrow < p.Sk ? p.S - 1 - q0 : -1;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int qc = c * 32 + i;
-            rs[i] = (qc >= first && qc <= last) ? rs[i] : 0xff800000u;      // -inf: probability 0
-          }
-        }
-        float pt[32], dst[32];
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int qc = c * 32 + i;
-          const float pr = fast_exp2(fmaf(__uint_as_float(rs[i]), sl2, -lse_b[qc]));
-          pt[i] = pr;
-          dst[i] = pr * (__uint_as_float(rp[i]) - dl_b[qc]);       // the softmax scale is applied once, to dK at the end
+            for (int i = 0; i < 32; ++i)
+              s[c][i] = (c * 32 + i >= first && c * 32 + i <= last) ? s[c][i] : 0xff800000u;   // -inf: probability 0
         }
-        // the P^T / dS^T tiles are single-buffered: the previous iteration's MMAs have to be done with them
-        if (c == 0 && it > 0 && !__all_sync(0xffffffffu, AT_WAIT(acc_done, (it - 1) & 1, 71))) { ok = false; break; }
-        store_row_chunk(sPT, t, c * 32, pt, p.is_bf16, AT_BM * 128);
-        store_row_chunk(sdST, t, c * 32, dst, p.is_bf16, AT_BM * 128);
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          const float4 n4 = nl[i / 4];
+          const uint32_t* v = &s[i >> 5][i & 31];
+          const float2 x = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2v, make_float2(n4.x, n4.y));
+          const float2 y = fma2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), sl2v, make_float2(n4.z, n4.w));
+          pr[i] = fast_exp2(x.x); pr[i + 1] = fast_exp2(x.y); pr[i + 2] = fast_exp2(y.x); pr[i + 3] = fast_exp2(y.y);
+          pk[i / 2] = pack2c<BF16>(pr[i], pr[i + 1]);
+          pk[i / 2 + 1] = pack2c<BF16>(pr[i + 2], pr[i + 3]);
+        }
+        tmem_st_32x32b_x32(tSh, pk);
       }
-      if (!ok) break;
+      tmem_st_wait();
       tc_fence_before_sync();
-      fence_proxy_async_smem();
+      mbar_arrive(p_ready);
+      if (!(ok = AT_WAIT_ALL(dp_full, it & 1, 72))) break;
+      tc_fence_after_sync();
+      uint32_t dp[2][32], ds[32];
+      tmem_ld_32x32b_x32(tdPh, dp[0]);
+      tmem_ld_32x32b_x32(tdPh + 32, dp[1]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 64; i += 4) {       // (the softmax scale is applied once, to dK at the end)
+        const float4 n4 = nd[i / 4];
+        const uint32_t* v = &dp[i >> 5][i & 31];
+        const float2 x = mul2(make_float2(pr[i], pr[i + 1]),
+                              add2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), make_float2(n4.x, n4.y)));
+        const float2 y = mul2(make_float2(pr[i + 2], pr[i + 3]),
+                              add2(make_float2(__uint_as_float(v[2]), __uint_as_float(v[3])), make_float2(n4.z, n4.w)));
+        ds[i / 2] = pack2c<BF16>(x.x, x.y);
+        ds[i / 2 + 1] = pack2c<BF16>(y.x, y.y);
+      }
+      tmem_st_32x32b_x32(tdPh, ds);
+      tmem_st_wait();
+      tc_fence_before_sync();
       mbar_arrive(ds_ready);
-      if (it + 1 < n_it) park_stats(it + 1, nxt);
-      __syncwarp();
     }
+    // the first warpgroup writes dV, the second dK
     const size_t orow = (((size_t)b * p.Sk + kvrow) * p.Hkv + kvh) * D;
     const bool valid = kvrow < p.Sk;
+    uint16_t* out = reinterpret_cast<uint16_t*>(half ? p.dk : p.dv) + orow;
+    const uint32_t src = (half ? tdK : tdV) + lane_base;
+    const float mul = half ? p.scale : 1.f;
     if (n_it == 0) {
       // no query row sees this kv tile: its gradient is zero (only the owning-store path has to write it)
-      if (ws == nullptr && valid) {
-        uint4 z = make_uint4(0, 0, 0, 0);
-        uint4* a = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.dk) + orow);
-        uint4* c = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.dv) + orow);
-        for (int i = 0; i < D / 8; ++i) { a[i] = z; c[i] = z; }
-      }
-    } else if (ok && __all_sync(0xffffffffu, AT_WAIT(acc_done, (n_it - 1) & 1, 72))) {
+      if (ws == nullptr && valid)
+        for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(out)[i] = make_uint4(0, 0, 0, 0);
+    } else if (ok && AT_WAIT_ALL(acc_done, 0, 73)) {
       tc_fence_after_sync();
       if (ws == nullptr) {
-        const int dt = p.is_bf16 ? DT_BF16 : DT_F16;
-        store_out_row(reinterpret_cast<uint16_t*>(p.dv) + orow, tdV + lane_base, D, valid, dt);
-        store_out_row(reinterpret_cast<uint16_t*>(p.dk) + orow, tdK + lane_base, D, valid, dt, p.scale);
+        store_out_row(out, src, D, valid, BF16 ? DT_BF16 : DT_F16, mul);
       } else {
         // ws = [2][B, Sk, Hkv, D] fp32: dK first, dV second
-        const size_t half = (size_t)p.B * p.Sk * p.Hkv * D;
+        float* dst = ws + (half ? 0 : (size_t)p.B * p.Sk * p.Hkv * D) + orow;
 #pragma unroll 1
-        for (int which = 0; which < 2; ++which) {
-          float* dst = ws + (which ? half : 0) + orow;
-          const uint32_t src = (which ? tdV : tdK) + lane_base;
-          const float mul = which ? 1.f : p.scale;
-#pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x32(src + c, r);
-            tmem_ld_wait();
-            if (valid) {
+        for (int c = 0; c < D; c += 32) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(src + c, v);
+          tmem_ld_wait();
+          if (valid) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 4)
-                atomicAdd(reinterpret_cast<float4*>(dst + c + i),
-                          make_float4(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul,
-                                      __uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul));
-            }
+            for (int i = 0; i < 32; i += 4)
+              atomicAdd(reinterpret_cast<float4*>(dst + c + i),
+                        make_float4(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul,
+                                    __uint_as_float(v[i + 2]) * mul, __uint_as_float(v[i + 3]) * mul));
           }
         }
       }
@@ -445,35 +486,39 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 4) { tc_fence_after_sync(); tmem_dealloc(tmem, TCOLS); }
+  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
 }
 
-// delta[b, h, s] = sum_d dO * O ; D / 8 lanes per row, 16 bytes per lane
+// Row statistics of the backward kernels, rows padded to whole q tiles: stats[0][b, h, s] = -lse in the log2 domain (-inf
+// behind the last row: probability 0), stats[1][b, h, s] = -sum_d dO * O.  D / 8 lanes per row, 16 bytes per lane.
 template <typename T, int D>
-__global__ void attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __restrict__ delta,
-                                  int B, int S, int H) {
+__global__ void attn_stats_kernel(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
+                                  float* __restrict__ stats, int B, int S, int Spad, int H) {
   constexpr int LPR = D / 8;                 // lanes per row (8 or 16)
-  const long long rows = (long long)B * S * H;
+  const long long rows = (long long)B * Spad * H;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
   const int sub = (int)(tid % LPR);
   // whole warps leave the loop together: rows per pass is a multiple of the rows a warp covers
   for (long long r0 = tid / LPR; r0 - (threadIdx.x & 31) / LPR < rows; r0 += nthreads / LPR) {
+    const int h = (int)(r0 % H);
+    const long long bs = r0 / H;
+    const int s = (int)(bs % Spad), b = (int)(bs / Spad);
+    const bool live = r0 < rows && s < S;
     float acc = 0.f;
-    if (r0 < rows) {
-      const Vec16<T> a = ld16(o + r0 * D + sub * 8);
-      const Vec16<T> g = ld16(dout + r0 * D + sub * 8);
+    if (live) {
+      const long long at = (((long long)b * S + s) * H + h) * D + sub * 8;
+      const Vec16<T> a = ld16(o + at);
+      const Vec16<T> g = ld16(dout + at);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc += Cvt<T>::to_f(a.v[i]) * Cvt<T>::to_f(g.v[i]);
     }
 #pragma unroll
     for (int m = LPR / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
     if (sub == 0 && r0 < rows) {
-      const int h = (int)(r0 % H);
-      const long long bs = r0 / H;
-      const int s_ = (int)(bs % S);
-      const int b = (int)(bs / S);
-      delta[((long long)b * H + h) * S + s_] = acc;
+      const long long at = ((long long)b * H + h) * Spad + s;
+      stats[at] = live ? -lse[((long long)b * H + h) * S + s] * LOG2E : -INFINITY;
+      stats[rows + at] = live ? -acc : 0.f;
     }
   }
 }
@@ -496,22 +541,40 @@ __global__ void attn_dkv_convert_kernel(const float* __restrict__ ws, T* __restr
   }
 }
 
-template <int D, int NCTA>
-static int launch_bwd(const CUtensorMap& tq128, const CUtensorMap& tdo128, const CUtensorMap& tk64,
-                      const CUtensorMap& tv64, const CUtensorMap& tq64, const CUtensorMap& tdo64,
-                      const CUtensorMap& tk128, const CUtensorMap& tv128, const AttnParams& p, float* ws,
-                      cudaStream_t st) {
-  // no alignment pad: shared memory of a CTA starts 1024-aligned (checked in the kernels), and at D = 64 two
-  // CTAs have to fit in one SM
-  const int smem_dq = 2 * AT_BM * D * 2 + 2 * BW_ST * BW_C * D * 2 + 128;
-  const int smem_kv = 2 * AT_BM * D * 2 + 2 * KV_ST * BW_C * D * 2 + 2 * AT_BM * BW_C * 2 + 16 * BW_C * 4 + 128;
+// Into how many parts a KV head's group of query heads is split in the dK/dV kernel: the fewest with which the longest CTA
+// takes at most a quarter longer than an even share of all tiles.  Whole groups (1) store their result directly; more
+// parts need the zeroed workspace, atomics and a conversion.
+static int dkdv_splits(int B, int S, int Sk, int Hq, int Hkv, int causal) {
+  const long long nq = (S + AT_BM - 1) / AT_BM, nk = (Sk + AT_BN - 1) / AT_BN;
+  const int group = Hq / Hkv;
+  const long long pairs = causal ? nq * (nk - nq) + nq * (nq + 1) / 2 : nq * nk;
+  const long long total = pairs * Hq * B;
+  for (int n = 1; n < group; ++n)
+    if (4 * (long long)sm_count() * nq * ((group + n - 1) / n) <= 5 * total) return n;
+  return group;
+}
+
+template <typename T, int D, bool BF16>
+static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                      const AttnParams& p, const void* o, const void* dout, const float* lse, float* stats, float* ws,
+                      int splits, cudaStream_t st) {
+  using C = BwdCfg<D>;
   static unsigned long long cfg_dq = 0, cfg_kv = 0;
   int r;
-  if ((r = smem_opt_in(attn_bwd_dq_kernel<D, NCTA>, smem_dq, cfg_dq)) != 0) return r;
-  if ((r = smem_opt_in(attn_bwd_dkdv_kernel<D, NCTA>, smem_kv, cfg_kv)) != 0) return r;
-  dim3 gq((p.S + AT_BM - 1) / AT_BM, p.Hq, p.B), gk((p.Sk + AT_BM - 1) / AT_BM, p.Hq, p.B);
-  attn_bwd_dq_kernel<D, NCTA><<<gq, 160, smem_dq, st>>>(tq128, tk64, tv64, tdo128, p);
-  attn_bwd_dkdv_kernel<D, NCTA><<<gk, 160, smem_kv, st>>>(tq64, tk128, tv128, tdo64, p, ws);
+  if ((r = smem_opt_in(attn_bwd_dq_kernel<D, BF16>, C::SMEM_DQ, cfg_dq)) != 0) return r;
+  if ((r = smem_opt_in(attn_bwd_dkdv_kernel<D, BF16>, C::SMEM_KV, cfg_kv)) != 0) return r;
+  const long long gq = (long long)((p.S + AT_BM - 1) / AT_BM) * p.Hq * p.B;
+  const long long gk = (long long)((p.Sk + AT_BM - 1) / AT_BM) * p.Hkv * splits * p.B;
+  if (gq > 0x7fffffff || gk > 0x7fffffff) return -5;
+  const long long lanes = (long long)p.B * p.Spad * p.Hq * (D / 8), nkv = (long long)p.B * p.Sk * p.Hkv * D;
+  attn_stats_kernel<T, D><<<gb_grid(lanes, 256), 256, 0, st>>>((const T*)o, (const T*)dout, lse, stats, p.B, p.S,
+                                                               p.Spad, p.Hq);
+  if (splits > 1 && (r = (int)cudaMemsetAsync(ws, 0, 2 * nkv * sizeof(float), st)) != 0) return r;
+  attn_bwd_dkdv_kernel<D, BF16><<<(int)gk, BW_THREADS, C::SMEM_KV, st>>>(tq, tk, tv, tdo, p, splits > 1 ? ws : nullptr,
+                                                                        splits);
+  attn_bwd_dq_kernel<D, BF16><<<(int)gq, BW_THREADS, C::SMEM_DQ, st>>>(tq, tk, tv, tdo, p);
+  if (splits > 1)
+    attn_dkv_convert_kernel<T><<<gb_grid(nkv / 2, 256), 256, 0, st>>>(ws, (T*)p.dk, (T*)p.dv, nkv);
   return (int)cudaGetLastError();
 }
 
@@ -519,47 +582,35 @@ static int launch_bwd(const CUtensorMap& tq128, const CUtensorMap& tdo128, const
 
 using namespace gb;
 
-// dkv_ws: fp32 scratch of 2 * B * Sk * Hkv * D elements, needed (and used) only when Hq != Hkv.
+// Into how many parts the query heads of a group are split (see dkdv_splits).
+extern "C" int gb_attn_bwd_splits(int B, int S, int Sk, int Hq, int Hkv, int causal) {
+  return dkdv_splits(B, S, Sk, Hq, Hkv, causal);
+}
+
+// scratch (fp32, 16-byte aligned): 2 * B * Hq * (S rounded up to 128) row statistics, and behind them
+// 2 * B * Sk * Hkv * D elements for dK and dV where gb_attn_bwd_splits() > 1.
 extern "C" int gb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                           const float* lse, float* delta, void* dq, void* dk, void* dv, float* dkv_ws, int B,
+                           const float* lse, float* scratch, void* dq, void* dk, void* dv, int B,
                            int S, int Sk, int Hq, int Hkv, int D, int causal, float scale, int is_bf16,
                            int* status, cudaStream_t st) {
   if (D != 64 && D != 128) return -2;
   if (Hq % Hkv != 0 || Sk < S) return -3;
-  const bool gqa = Hq != Hkv;
-  if (gqa && dkv_ws == nullptr) return -4;
-  CUtensorMap tq, tk, tv, tdo, tq64, tk64, tv64, tdo64;
+  if (scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return -4;
+  CUtensorMap tq, tk, tv, tdo;
   int r;
-  if ((r = make_tmap_bshd(&tq, q, is_bf16, B, S, Hq, D, 128)) != 0) return 10000 + r;
-  if ((r = make_tmap_bshd(&tk, k, is_bf16, B, Sk, Hkv, D, 128)) != 0) return 20000 + r;
-  if ((r = make_tmap_bshd(&tv, v, is_bf16, B, Sk, Hkv, D, 128)) != 0) return 30000 + r;
-  if ((r = make_tmap_bshd(&tdo, dout, is_bf16, B, S, Hq, D, 128)) != 0) return 40000 + r;
-  if ((r = make_tmap_bshd(&tq64, q, is_bf16, B, S, Hq, D, BW_C)) != 0) return 50000 + r;
-  if ((r = make_tmap_bshd(&tk64, k, is_bf16, B, Sk, Hkv, D, BW_C)) != 0) return 60000 + r;
-  if ((r = make_tmap_bshd(&tv64, v, is_bf16, B, Sk, Hkv, D, BW_C)) != 0) return 70000 + r;
-  if ((r = make_tmap_bshd(&tdo64, dout, is_bf16, B, S, Hq, D, BW_C)) != 0) return 80000 + r;
-  const long long rows = (long long)B * S * Hq;
-  const int dgrid = gb_grid(rows * (D / 8), 256);
-  if (is_bf16 && D == 64) attn_delta_kernel<__nv_bfloat16, 64><<<dgrid, 256, 0, st>>>(
-      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, Hq);
-  else if (is_bf16) attn_delta_kernel<__nv_bfloat16, 128><<<dgrid, 256, 0, st>>>(
-      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, Hq);
-  else if (D == 64) attn_delta_kernel<__half, 64><<<dgrid, 256, 0, st>>>((const __half*)o, (const __half*)dout,
-                                                                        delta, B, S, Hq);
-  else attn_delta_kernel<__half, 128><<<dgrid, 256, 0, st>>>((const __half*)o, (const __half*)dout, delta, B, S, Hq);
-  const long long nkv = (long long)B * Sk * Hkv * D;
-  if (gqa && (r = (int)cudaMemsetAsync(dkv_ws, 0, 2 * nkv * sizeof(float), st)) != 0) return r;
+  if ((r = make_tmap_bshd(&tq, q, is_bf16, B, S, Hq, D)) != 0) return 10000 + r;
+  if ((r = make_tmap_bshd(&tk, k, is_bf16, B, Sk, Hkv, D)) != 0) return 20000 + r;
+  if ((r = make_tmap_bshd(&tv, v, is_bf16, B, Sk, Hkv, D)) != 0) return 30000 + r;
+  if ((r = make_tmap_bshd(&tdo, dout, is_bf16, B, S, Hq, D)) != 0) return 40000 + r;
   AttnParams p{};
-  p.lse_in = lse; p.delta = delta; p.dq = dq; p.dk = dk; p.dv = dv; p.status = status;
+  p.Spad = (S + AT_BM - 1) / AT_BM * AT_BM;
+  p.stats = scratch; p.dq = dq; p.dk = dk; p.dv = dv; p.status = status;
   p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal; p.is_bf16 = is_bf16; p.scale = scale;
-  float* ws = gqa ? dkv_ws : nullptr;
-  if (D == 64) r = launch_bwd<64, 2>(tq, tdo, tk64, tv64, tq64, tdo64, tk, tv, p, ws, st);
-  else r = launch_bwd<128, 1>(tq, tdo, tk64, tv64, tq64, tdo64, tk, tv, p, ws, st);
-  if (r != 0) return r;
-  if (gqa) {
-    if (is_bf16) attn_dkv_convert_kernel<__nv_bfloat16><<<gb_grid(nkv / 2, 256), 256, 0, st>>>(
-        dkv_ws, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, nkv);
-    else attn_dkv_convert_kernel<__half><<<gb_grid(nkv / 2, 256), 256, 0, st>>>(dkv_ws, (__half*)dk, (__half*)dv, nkv);
-  }
-  return (int)cudaGetLastError();
+  float* ws = scratch + 2 * (long long)B * Hq * p.Spad;
+  const int splits = dkdv_splits(B, S, Sk, Hq, Hkv, causal);
+  if (D == 64)
+    return is_bf16 ? launch_bwd<__nv_bfloat16, 64, true>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st)
+                   : launch_bwd<__half, 64, false>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st);
+  return is_bf16 ? launch_bwd<__nv_bfloat16, 128, true>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st)
+                 : launch_bwd<__half, 128, false>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st);
 }

@@ -13,7 +13,7 @@ constexpr float LN2 = 0.6931471805599453f;
 
 struct AttnParams {
   void* o; float* lse;                       // forward outputs
-  const float* lse_in; const float* delta;   // backward inputs
+  const float* stats; int Spad;              // backward input: padded row statistics [2][B, Hq, Spad]
   void* dq; void* dk; void* dv;              // backward outputs
   int* status;
   int B, S, Sk, Hq, Hkv;
@@ -21,8 +21,8 @@ struct AttnParams {
   float scale;                               // softmax scale
 };
 
-// 32 fp32 values of row `row`, columns c0..c0+31, into a K-major 128-byte-swizzled 16-bit tile whose
-// 64-column chunks are `chunk_stride` bytes apart (the layout TMA SWIZZLE_128B produces).
+// 32 fp32 values of row `row` as 16-bit units u0..u0+3 (16 bytes each) of a 128-byte-swizzled row at `base` (the layout
+// TMA SWIZZLE_128B reads and writes).
 template <bool BF16>
 __device__ __forceinline__ void store_row_chunk_t(uint8_t* base, int u0, int row, const float (&v)[32]) {
 #pragma unroll
@@ -34,13 +34,6 @@ __device__ __forceinline__ void store_row_chunk_t(uint8_t* base, int u0, int row
     w.w = pack2c<BF16>(v[i * 8 + 6], v[i * 8 + 7]);
     *reinterpret_cast<uint4*>(base + (((u0 + i) ^ (row & 7)) << 4)) = w;
   }
-}
-__device__ __forceinline__ void store_row_chunk(uint8_t* tile, int row, int c0, const float (&v)[32], int is_bf16,
-                                                int chunk_stride) {
-  uint8_t* base = tile + (c0 >> 6) * chunk_stride + row * 128;
-  const int u0 = (c0 & 63) >> 3;
-  if (is_bf16) store_row_chunk_t<true>(base, u0, row, v);
-  else store_row_chunk_t<false>(base, u0, row, v);
 }
 
 // K-major operand (contraction inside the 128-byte rows): k-step kk of 16 elements

@@ -15,13 +15,6 @@ constexpr int RS_THREADS = 256;
 constexpr int RS_MIN_ROW_BYTES = 8192;        // below this the register-resident kernels have enough rows in flight
 constexpr int RS_MAX_ROW_BYTES = 65536;
 
-// `bytes` from global to shared memory (both 16-byte aligned, bytes a multiple of 16), completion posted on `bar`
-__device__ __forceinline__ void rs_bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
 template <typename T, typename Op>
 __global__ void __launch_bounds__(RS_THREADS)
 row_stream_kernel(const T* __restrict__ x, long long rows, int cols, Op op, int* __restrict__ status) {
@@ -44,7 +37,7 @@ row_stream_kernel(const T* __restrict__ x, long long rows, int cols, Op op, int*
       const long long r = blockIdx.x + s * stride;
       if (r < rows) {
         mbar_expect_tx(&full[s], row_bytes);
-        rs_bulk_load(rs_smem + (size_t)s * row_bytes, x + r * cols, row_bytes, &full[s]);
+        bulk_load(rs_smem + (size_t)s * row_bytes, x + r * cols, row_bytes, &full[s]);
       }
     }
   }
@@ -66,7 +59,7 @@ row_stream_kernel(const T* __restrict__ x, long long rows, int cols, Op op, int*
     const long long nxt = r + 2 * stride;
     if (threadIdx.x == 0 && nxt < rows) {
       mbar_expect_tx(&full[s], row_bytes);
-      rs_bulk_load(rs_smem + (size_t)s * row_bytes, x + nxt * cols, row_bytes, &full[s]);
+      bulk_load(rs_smem + (size_t)s * row_bytes, x + nxt * cols, row_bytes, &full[s]);
     }
   }
 }

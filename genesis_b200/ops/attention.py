@@ -10,9 +10,11 @@ import torch
 from . import native as N
 
 _SIG_FWD = "ppppp" + "iiiiii" + "i" + "f" + "i" + "pp"
-_SIG_BWD = "ppppppppppp" + "iiiiii" + "i" + "f" + "i" + "pp"
+_SIG_SPLITS = "iiiiii"
+_SIG_BWD = "pppppppppp" + "iiiiii" + "i" + "f" + "i" + "pp"
 N._SIGS["gb_attn_fwd"] = _SIG_FWD
 N._SIGS["gb_attn_bwd"] = _SIG_BWD
+N._SIGS["gb_attn_bwd_splits"] = _SIG_SPLITS
 _bound = False
 
 
@@ -20,7 +22,8 @@ def _lib():
     global _bound
     L = N.lib()
     if not _bound:
-        for name, sig in (("gb_attn_fwd", _SIG_FWD), ("gb_attn_bwd", _SIG_BWD)):
+        for name, sig in (("gb_attn_fwd", _SIG_FWD), ("gb_attn_bwd", _SIG_BWD),
+                          ("gb_attn_bwd_splits", _SIG_SPLITS)):
             fn = getattr(L, name)
             fn.argtypes = [N._C[c] for c in sig]
             fn.restype = ctypes.c_int
@@ -58,12 +61,14 @@ def backward(do, q, k, v, o, lse, causal, scale):
     B, S, Hq, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    delta = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
-    # grouped-query attention: the query heads of a group accumulate dK / dV in fp32 scratch
-    ws = torch.empty(2 * k.numel(), dtype=torch.float32, device=q.device) if Hq != Hkv else None
-    N._chk(_lib().gb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-                              delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                              ws.data_ptr() if ws is not None else None, B, S, Sk, Hq, Hkv, D,
+    # row statistics, and an fp32 dK / dV workspace where the query heads of a group are shared out between CTAs
+    L = _lib()
+    n = 2 * B * Hq * (-(-S // 128) * 128)
+    if L.gb_attn_bwd_splits(B, S, Sk, Hq, Hkv, 1 if causal else 0) > 1:
+        n += 2 * k.numel()
+    scratch = torch.empty(n, dtype=torch.float32, device=q.device)
+    N._chk(L.gb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                              scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, Sk, Hq, Hkv, D,
                               1 if causal else 0, float(scale), 1 if q.dtype == torch.bfloat16 else 0,
                               N.status_tensor(q.device).data_ptr(), N._st()), "attn_bwd")
     return dq, dk, dv

@@ -1,5 +1,5 @@
 """The attention kernels at the edges of their tiles, work items and routes: 128-row and 128-column tiles, pairs of q
-tiles, groups of query rows that the decoding kernel takes, kv tiles that few queries see, and scores whose maximum keeps
+tiles, kv tiles that few queries see, and scores whose maximum keeps
 growing (the accumulator's rescaling).  The oracle is the softmax in float64."""
 import math
 
@@ -74,3 +74,32 @@ def test_forward_at_tile_edges(case, dt, causal):
 @pytest.mark.parametrize("ramp", [60.0, -60.0])
 def test_forward_with_growing_scores(shape, ramp):
     _check_fwd(*_inputs(*shape, torch.bfloat16, ramp=ramp), True)
+
+
+BWD = [
+    (1, 127, 127, 2, 1, 64), (1, 129, 130, 4, 2, 128), (2, 256, 256, 6, 3, 64), (1, 385, 500, 14, 2, 64),
+    (1, 40, 700, 4, 1, 128), (4, 520, 520, 12, 2, 128), (8, 650, 650, 14, 2, 64), (2, 384, 384, 5, 5, 128),
+    (1, 1, 1, 2, 1, 64), (1, 3, 260, 6, 2, 128),
+]
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("case", BWD)
+@pytest.mark.parametrize("causal", [True, False])
+def test_backward_at_tile_edges(case, dt, causal):
+    q, k, v = _inputs(*case, dt)
+    o, lse, scale = _check_fwd(q, k, v, causal)
+    do = torch.randn(q.shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).to(dt)
+    r = N.attention_bwd(do, q, k, v, o, lse, causal, scale)
+    assert r is not NotImplemented
+    N.check_status()
+    leaves = [t.double().requires_grad_() for t in (q, k, v)]
+    _oracle(*leaves, causal, scale)[0].backward(do.double())
+    # P and dS are rounded once to 16 bits, delta carries the rounding of o, the result is rounded once: four independent
+    # roundings of relative error up to u (2^-8 or 2^-11, as above), u / sqrt(3) in the norm each, so 2 u; the floor is what fp32 leaves of dP - delta where
+    # the two cancel (D products of up to 20 at 2^-24 each, over a few hundred elements)
+    u = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    for got, ref in zip(r, leaves):
+        ref = ref.grad
+        assert float((got.double() - ref).norm()) <= 2 * u * float(ref.norm()) + 1e-3
+        assert bool(torch.isfinite(got).all())
