@@ -99,4 +99,7 @@ static inline int make_tmap_bshd(CUtensorMap* out, const void* base, int is_bf16
 
 
 
+// attention of a few query rows (attention_decode_sm100.cu); arguments as checked by gb_attn_fwd
+int attn_decode(const void* q, const void* k, const void* v, const AttnParams& p, int D, cudaStream_t st);
+
 }  // namespace gb

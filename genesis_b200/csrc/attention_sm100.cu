@@ -370,6 +370,16 @@ extern "C" int gb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   AttnParams p{};
   p.o = o; p.lse = lse; p.status = status; p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
   p.causal = causal; p.is_bf16 = is_bf16; p.scale = scale;
+  // A few query rows: the decoding kernel reads K and V once per 16 rows of a group and splits the keys, the tiled kernel
+  // reads them once per head and does not.  Up to 16 rows it always wins (107 -> 19 us for 8 x 1 queries, 32 / 4 heads of
+  // 128, 4096 keys; 8.4 -> 6.8 us for one query and 64 keys).  Up to 64 it does where it reads no more often than the
+  // tiled kernel (64 x 8 queries, 32 / 4 heads, 1024 keys: 83 us against 244) or where the tiled grid leaves half the GPU idle
+  // (8 x 64, 4 / 4 heads, 4096 keys: 29 against 58), and loses elsewhere (64 x 64, 4 / 4 heads, 1024 keys: 55 against 27)
+  // and on short keys (8 queries, 32 / 4 heads, 64 keys: 9.8 against 8.4).
+  const long long rows = (long long)S * (Hq / Hkv), passes = (rows + 15) / 16;
+  if ((rows <= 16 || (rows <= 64 && Sk >= 256 && (passes <= Hq / Hkv || 2ll * B * Hq <= sm_count()))) && B <= 65535 &&
+      4 * Hkv <= 65535)
+    return attn_decode(q, k, v, p, D, st);
   CUtensorMap tq, tk, tv, to;
   int r;
   if ((r = make_tmap_bshd(&tq, q, is_bf16, B, S, Hq, D)) != 0) return 10000 + r;

@@ -1,5 +1,5 @@
 """The attention kernels at the edges of their tiles, work items and routes: 128-row and 128-column tiles, pairs of q
-tiles, kv tiles that few queries see, and scores whose maximum keeps
+tiles, groups of query rows that the decoding kernel takes, kv tiles that few queries see, and scores whose maximum keeps
 growing (the accumulator's rescaling).  The oracle is the softmax in float64."""
 import math
 
@@ -60,6 +60,9 @@ FWD = [
     # B, S, Sk, Hq, Hkv, D: one tile and its neighbours, one row more than a pair, ragged keys, enough work for pairs
     (1, 127, 127, 2, 1, 64), (1, 129, 129, 9, 3, 64), (1, 255, 300, 2, 2, 128), (2, 257, 257, 4, 2, 128),
     (1, 385, 1000, 14, 2, 64), (3, 640, 640, 40, 8, 64), (2, 513, 513, 80, 16, 128), (40, 130, 131, 4, 4, 64),
+    # a few query rows: one, a full 16-row tile, one more, the largest that the decoding kernel takes, and the first past it
+    (1, 1, 1, 1, 1, 64), (2, 1, 17, 8, 1, 128), (3, 2, 1030, 16, 2, 64), (1, 17, 100, 1, 1, 128), (2, 5, 4099, 12, 2, 128),
+    (1, 64, 64, 2, 2, 64), (1, 65, 65, 2, 2, 64), (9, 1, 513, 32, 4, 128), (1, 4, 333, 64, 4, 64),
 ]
 
 
@@ -70,7 +73,7 @@ def test_forward_at_tile_edges(case, dt, causal):
     _check_fwd(*_inputs(*case, dt), causal)
 
 
-@pytest.mark.parametrize("shape", [(1, 700, 700, 2, 1, 64), (1, 300, 900, 2, 2, 128)])
+@pytest.mark.parametrize("shape", [(1, 700, 700, 2, 1, 64), (1, 300, 900, 2, 2, 128), (2, 1, 2000, 8, 2, 64), (1, 3, 700, 4, 4, 128)])
 @pytest.mark.parametrize("ramp", [60.0, -60.0])
 def test_forward_with_growing_scores(shape, ramp):
     _check_fwd(*_inputs(*shape, torch.bfloat16, ramp=ramp), True)
