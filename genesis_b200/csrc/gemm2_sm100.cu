@@ -199,7 +199,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
   uint32_t* poison_slot = tmem_base_slot + 2;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (warp-uniform, and known to be)
   const uint32_t rank = cta_rank_in_cluster();          // 0 = leader
   const uint32_t peer = rank ^ 1u;
   const int cluster_id = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
@@ -297,38 +297,49 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
     }
     __syncwarp();
   } else if (warp == 1) {
-    // =========================== MMA issuer: one thread of the leader CTA ===========================
-    if (rank == 0 && lane == 0) {
+    // ====== MMA issuer of the leader CTA: the warp stays converged (its addresses live in uniform registers), one
+    // elected lane issues ======
+    if (rank == 0) {
       const uint32_t idesc = make_idesc(p.in_bf16 ? 1u : 0u, A_MN ? 1u : 0u, B_MN ? 1u : 0u, 2 * BM, p.bn);
       uint32_t it = 0, tile_no = 0;
-      for (long long t = cluster_id; t < total_tiles && !*abort_flag; t += nclusters) {
+      for (long long t = cluster_id; t < total_tiles; t += nclusters) {
         const uint32_t acc = tile_no & 1, acc_ph = (tile_no >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, 200)) { give_up(); break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, 200))) {
+          if (lane == 0) give_up();
+          break;
+        }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
         bool ok = true;
         for (int k0 = 0; k0 < p.K; k0 += BK, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, p.status, 201)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, abort_flag, p.status, 201))) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
           const uint32_t b_addr = a_addr + A_BYTES;
+          const uint64_t da = A_MN ? make_smem_desc(a_addr, BK * 128, 1024) : make_smem_desc(a_addr, 16, 1024);
+          const uint64_t db = B_MN ? make_smem_desc(b_addr, BK * 128, 1024) : make_smem_desc(b_addr, 16, 1024);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < KSTEPS; ++kk) {
-            const uint64_t da = A_MN ? make_smem_desc(a_addr + kk * UMMA_K * 128, BK * 128, 1024)
-                                     : make_smem_desc(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc(b_addr + kk * UMMA_K * 128, BK * 128, 1024)
-                                     : make_smem_desc(b_addr + kk * 32, 16, 1024);
-            umma2_f16(d_tmem, da, db, idesc, (k0 == 0 && kk == 0) ? 0u : 1u);
+            for (int kk = 0; kk < KSTEPS; ++kk)       // (descriptors count 16-byte units)
+              umma2_f16(d_tmem, da + (A_MN ? kk * UMMA_K * 128 : kk * 32) / 16, db + (B_MN ? kk * UMMA_K * 128 : kk * 32) / 16,
+                        idesc, (k0 == 0 && kk == 0) ? 0u : 1u);
+            // the stage is free in both CTAs once these MMAs have read it
+            umma2_commit(smem_u32(&empty_bar[s]));
+            umma2_commit(map_to_cta(smem_u32(&empty_bar[s]), 1));
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          umma2_commit(smem_u32(&empty_bar[s]));
-          umma2_commit(map_to_cta(smem_u32(&empty_bar[s]), 1));
+          __syncwarp();
         }
-        if (!ok) { give_up(); break; }
-        umma2_commit(smem_u32(&tmem_full[acc]));
-        umma2_commit(map_to_cta(smem_u32(&tmem_full[acc]), 1));
+        if (!ok) {
+          if (lane == 0) give_up();
+          break;
+        }
+        if (elect_one()) {
+          umma2_commit(smem_u32(&tmem_full[acc]));
+          umma2_commit(map_to_cta(smem_u32(&tmem_full[acc]), 1));
+        }
+        __syncwarp();
         ++tile_no;
       }
     }

@@ -100,7 +100,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ C
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
   int* s_offs = reinterpret_cast<int*>(tmem_base_slot + 4);   // up to 200 group offsets
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);     // warp-uniform, and known to be
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -232,18 +232,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ C
       }
     }
   } else if (warp == 1) {
-    // =========================== MMA issuer (one thread) ===========================
-    if (lane == 0) {
+    // ====== MMA issuer: the warp stays converged (its addresses live in uniform registers), one elected lane issues ======
+    // Building both descriptors anew for every instruction in a divergent branch took longer than the instruction: 171
+    // clocks per 128 x 256 x 16 MMA, 107 per 128 x 128 x 16; with descriptors advanced by constants they issue at the rate
+    // the pipe takes them, 128 and 64.  4096 cubed: 0.153 -> 0.132 ms; 8192 cubed: 0.867 -> 0.777; 16384 cubed: 7.48 -> 6.70;
+    // 16384 x 4864 x 896 (CTA pairs): 0.111 -> 0.100; 16384 x 151936 x 896: 4.00 -> 3.85.
+    {
       const uint32_t fmt = (ESIZE == 4) ? 2u : (uint32_t)(p.out_dtype >> 8);   // operand format rides in bits 8+
       const uint32_t idesc = make_idesc(fmt, A_MN ? 1u : 0u, B_MN ? 1u : 0u, BM, BN);
       uint32_t it = 0, tile_no = 0;
       long long cur = cur0;
       int mi, ni, z, k_begin, k_end;
-      while (!*abort_flag && advance(cur, mi, ni, z, k_begin, k_end)) {
+      while (advance(cur, mi, ni, z, k_begin, k_end)) {
         if (p.group_mode == GROUP_M && mi * BM >= s_offs[p.groups]) continue;
         const uint32_t acc = tile_no & 1;
         const uint32_t acc_ph = (tile_no >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, 200)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, 200))) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
         bool first = true;
@@ -251,26 +255,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ C
         for (int k0 = k_begin; k0 < k_end; k0 += BK, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&full_bar[s], ph, abort_flag, p.status, 201)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph, abort_flag, p.status, 201))) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
           const uint32_t b_addr = a_addr + L::A_BYTES;
+          const uint64_t da = A_MN ? make_smem_desc(a_addr, BK * BK_BYTES, 1024) : make_smem_desc(a_addr, 16, 1024);
+          const uint64_t db = B_MN ? make_smem_desc(b_addr, BK * BK_BYTES, 1024) : make_smem_desc(b_addr, 16, 1024);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < KSTEPS; ++kk) {
-            // K-major: advance 32 bytes inside the 128-byte swizzle row.
-            // MN-major: advance UMMA_K k-rows of 128 bytes.
-            const uint64_t da = A_MN ? make_smem_desc(a_addr + kk * UMMA_K * BK_BYTES, BK * BK_BYTES, 1024)
-                                     : make_smem_desc(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = B_MN ? make_smem_desc(b_addr + kk * UMMA_K * BK_BYTES, BK * BK_BYTES, 1024)
-                                     : make_smem_desc(b_addr + kk * 32, 16, 1024);
-            if constexpr (ESIZE == 4) umma_tf32(d_tmem, da, db, idesc, (first && kk == 0) ? 0u : 1u);
-            else umma_f16(d_tmem, da, db, idesc, (first && kk == 0) ? 0u : 1u);
+            for (int kk = 0; kk < KSTEPS; ++kk) {
+              // K-major: advance 32 bytes inside the 128-byte swizzle row.
+              // MN-major: advance UMMA_K k-rows of 128 bytes.  (descriptors count 16-byte units)
+              const uint32_t oa = (A_MN ? kk * UMMA_K * BK_BYTES : kk * 32) / 16;
+              const uint32_t ob = (B_MN ? kk * UMMA_K * BK_BYTES : kk * 32) / 16;
+              if constexpr (ESIZE == 4) umma_tf32(d_tmem, da + oa, db + ob, idesc, (first && kk == 0) ? 0u : 1u);
+              else umma_f16(d_tmem, da + oa, db + ob, idesc, (first && kk == 0) ? 0u : 1u);
+            }
+            umma_commit(&empty_bar[s]);   // frees the smem stage once these MMAs have read it
           }
-          umma_commit(&empty_bar[s]);   // frees the smem stage once these MMAs have read it
+          __syncwarp();
           first = false;
         }
         if (!ok) break;
-        umma_commit(&tmem_full[acc]);
+        if (elect_one()) umma_commit(&tmem_full[acc]);
+        __syncwarp();
         ++tile_no;
       }
     }
