@@ -156,7 +156,9 @@ __global__ void moe_scatter_kernel(const int* __restrict__ experts, const int* _
   }
 }
 
-// out[t, :] = sum_j w[t, j] * y[pos[t, j], :]
+// out[t, :] = sum_j w[t, j] * y[pos[t, j], :]; without `w` every weight is 1: the gradient of the row gather that
+// sorted the tokens, in a fixed order and without atomics (4096 tokens x 8 rows of 2048 bf16: 28 us; the scatter with
+// one fp32 atomic per element took 282 us, besides zeroing its buffer and converting it).
 template <typename T>
 __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ w, const int* __restrict__ pos,
                                    T* __restrict__ out, long long tokens, int k, int cols) {
@@ -171,7 +173,7 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
 #pragma unroll
     for (int j = 0; j < V; ++j) acc[j] = 0.f;
     for (int s = 0; s < k; ++s) {
-      const float ws = w[t * k + s];
+      const float ws = w != nullptr ? w[t * k + s] : 1.f;
       const Vec16<T> a = ld16(y + (long long)pos[t * k + s] * cols + c * V);
 #pragma unroll
       for (int j = 0; j < V; ++j) acc[j] += ws * Cvt<T>::to_f(a.v[j]);
@@ -184,6 +186,50 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
 }
 
 // backward of combine: dy[pos[t,j], :] = w[t,j] * g[t, :];  dw[t,j] = <g[t,:], y[pos[t,j],:]>
+// One warp per (token, slot), 16 bytes per lane: y is read and dy written once; the k warps of a token sit in one CTA,
+// so its row of g comes from L1 after the first of them.  4096 tokens x 8 x 2048 bf16: 91 us with two bytes per lane -> 49 us.
+template <typename T>
+__global__ void moe_combine_bwd_vec_kernel(const T* __restrict__ g, const T* __restrict__ y, const float* __restrict__ w,
+                                           const int* __restrict__ pos, T* __restrict__ dy, float* __restrict__ dw,
+                                           long long tokens, int k, int cols) {
+  constexpr int V = Vec16<T>::N;
+  const int lane = threadIdx.x & 31, nv = cols / V;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long pr = warp; pr < tokens * k; pr += nwarps) {
+    const T* gr = g + pr / k * cols;
+    const long long row = (long long)pos[pr] * cols;
+    const float ws = w[pr];
+    float dot = 0.f;
+#pragma unroll 4
+    for (int c = lane; c < nv; c += 32) {
+      const Vec16<T> a = ld16(gr + c * V), b = ld16(y + row + c * V);
+      Vec16<T> o;
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float gg = Cvt<T>::to_f(a.v[j]);
+        dot += gg * Cvt<T>::to_f(b.v[j]);
+        o.v[j] = Cvt<T>::from_f(ws * gg);
+      }
+      st16(dy + row + c * V, o);
+    }
+    dot = warp_sum(dot);
+    if (lane == 0) dw[pr] = dot;
+  }
+}
+
+// zeroes the rows of `dst` that no token was sorted into (row_token < 0); one warp per row
+__global__ void moe_zero_pads_kernel(const int* __restrict__ row_token, uint4* __restrict__ dst, long long rows,
+                                     int vec_per_row) {
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
+    if (row_token[r] >= 0) continue;
+    for (int c = lane; c < vec_per_row; c += 32) dst[r * vec_per_row + c] = make_uint4(0, 0, 0, 0);
+  }
+}
+
+// the same for rows that are not whole 16-byte vectors
 template <typename T>
 __global__ void moe_combine_bwd_kernel(const T* __restrict__ g, const T* __restrict__ y, const float* __restrict__ w,
                                        const int* __restrict__ pos, T* __restrict__ dy, float* __restrict__ dw,
@@ -255,9 +301,24 @@ extern "C" int gb_moe_combine(const void* y, const float* w, const int* pos, voi
   return (int)cudaGetLastError();
 }
 
-extern "C" int gb_moe_combine_bwd(const void* g, const void* y, const float* w, const int* pos, void* dy, float* dw,
-                                  long long tokens, int k, int cols, int dt, cudaStream_t st) {
-  if (tokens == 0) return 0;
+// dy has `rows` rows.  With `row_token` (negative where no token was sorted to) the rows without a token are zeroed here;
+// without it the caller has zeroed dy.
+extern "C" int gb_moe_combine_bwd(const void* g, const void* y, const float* w, const int* pos, const int* row_token,
+                                  void* dy, float* dw, long long tokens, long long rows, int k, int cols, int dt,
+                                  cudaStream_t st) {
+  const int es = dt == DT_F32 ? 4 : 2;
+  const bool vec = (long long)cols * es % 16 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
+  if (row_token != nullptr && rows > 0) {
+    if (!vec) return -2;
+    moe_zero_pads_kernel<<<gb_grid(rows * 32, 256), 256, 0, st>>>(row_token, (uint4*)dy, rows, cols * es / 16);
+  }
+  if (tokens == 0) return (int)cudaGetLastError();
+  if (vec) {
+    GB_DISPATCH_FLOAT(dt, T, moe_combine_bwd_vec_kernel<T><<<gb_grid(tokens * k * 32, 256), 256, 0, st>>>(
+        (const T*)g, (const T*)y, w, pos, (T*)dy, dw, tokens, k, cols));
+    return (int)cudaGetLastError();
+  }
   GB_DISPATCH_FLOAT(dt, T, moe_combine_bwd_kernel<T><<<gb_grid(tokens * k * 32, 256), 256, 0, st>>>(
       (const T*)g, (const T*)y, w, pos, (T*)dy, dw, tokens, k, cols));
   return (int)cudaGetLastError();

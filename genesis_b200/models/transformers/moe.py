@@ -192,19 +192,22 @@ class GroupedExpertsFunction(Function):
 
 
 class DispatchFunction(Function):
-    """Row gather into expert-sorted order: out[i] = x[token_of[i]]; backward scatter-adds."""
+    """Row gather into expert-sorted order: out[i] = x[token_of[i]].  Backward sums every token's rows, found through
+    `pos` (the sorted row of each (token, slot)) or, without it, scatter-added."""
     raw = True
     amp_policy = AMPPolicy.PRESERVE
 
     @staticmethod
-    def forward(ctx, x, token_of):
-        ctx.save_for_backward(token_of)
+    def forward(ctx, x, token_of, pos=None):
+        ctx.save_for_backward(token_of, pos)
         ctx.n = x.shape[0]
         return K.gather_rows(x, token_of)
 
     @staticmethod
     def backward(ctx, g):
-        (token_of,) = ctx.saved_tensors
+        token_of, pos = ctx.saved_tensors
+        if pos is not None:
+            return K.moe_gather_sum(g if g.is_contiguous() else K.contiguous(g), pos)
         return K.scatter_add_rows(g, token_of, ctx.n, g.dtype)
 
 
@@ -214,15 +217,15 @@ class CombineFunction(Function):
     amp_policy = AMPPolicy.PRESERVE
 
     @staticmethod
-    def forward(ctx, y, w, pos):
-        ctx.save_for_backward(y, w, pos)
+    def forward(ctx, y, w, pos, token_of=None):
+        ctx.save_for_backward(y, w, pos, token_of)
         return K.moe_combine(y, w, pos)
 
     @staticmethod
     def backward(ctx, g):
-        y, w, pos = ctx.saved_tensors
+        y, w, pos, token_of = ctx.saved_tensors
         g = g if g.dtype == y.dtype else K.to_dtype(g, y.dtype)
-        dy, dw = K.moe_combine_bwd(g if g.is_contiguous() else K.contiguous(g), y, w, pos)
+        dy, dw = K.moe_combine_bwd(g if g.is_contiguous() else K.contiguous(g), y, w, pos, token_of)
         return dy, dw.to(w.dtype)
 
 
@@ -335,9 +338,10 @@ class MoELayer(Module):
 
     def _local_forward(self, x, idx, w):
         token_of, pos, offsets = K.moe_sort(idx, self.num_experts)
-        xs = DispatchFunction.apply(x, Tensor._wrap(token_of))
+        token_of, pos = Tensor._wrap(token_of), Tensor._wrap(pos)
+        xs = DispatchFunction.apply(x, token_of, pos)
         ys = self.experts(xs, offsets)
-        return CombineFunction.apply(ys, w, Tensor._wrap(pos))
+        return CombineFunction.apply(ys, w, pos, token_of)
 
 
 # ------------------------------------------------------------------------------------

@@ -1049,10 +1049,22 @@ def moe_combine(y, w, pos):
     return (rows.float() * w.float().unsqueeze(-1)).sum(1).to(y.dtype)
 
 
-def moe_combine_bwd(g, y, w, pos):
-    """Returns (dy [like y, zero in rows no pair points to], dw [T, k] fp32)."""
+def moe_gather_sum(y, pos):
+    """out[t] = sum_j y[pos[t, j]] (fp32 sum): the gradient of the gather that sorted the tokens."""
     if y.is_cuda:
-        r = N.moe_combine_bwd(g, y, w, pos)
+        r = N.moe_gather_sum(y, pos)
+        if r is not NotImplemented:
+            return r
+        _fell("moe_gather_sum")
+    T, k = pos.shape
+    return y.index_select(0, pos.reshape(-1).long()).reshape(T, k, -1).float().sum(1).to(y.dtype)
+
+
+def moe_combine_bwd(g, y, w, pos, token_of=None):
+    """Returns (dy [like y, zero in rows no pair points to], dw [T, k] fp32).  `token_of` (negative in rows without a
+    token), where the caller has it, saves zeroing the rows that are overwritten."""
+    if y.is_cuda:
+        r = N.moe_combine_bwd(g, y, w, pos, token_of)
         if r is not NotImplemented:
             return r
         _fell("moe_combine_bwd")

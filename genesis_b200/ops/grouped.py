@@ -112,14 +112,33 @@ def moe_combine(y, w, pos):
     return out
 
 
-def moe_combine_bwd(g, y, w, pos):
+def moe_gather_sum(y, pos):
+    """out[t] = sum_j y[pos[t, j]], fp32 sum."""
+    if y.dtype not in N._FLOATS or not y.is_contiguous() or y.data_ptr() % 16 or pos.dtype != torch.int32:
+        return NotImplemented
+    T, k = pos.shape
+    out = torch.empty(T, y.shape[1], dtype=y.dtype, device=y.device)
+    rc = N.lib().gb_moe_combine(y.data_ptr(), None, pos.contiguous().data_ptr(), out.data_ptr(), T, k, y.shape[1],
+                                N._DT[y.dtype], N._st())
+    if rc == -2:
+        return NotImplemented
+    N._chk(rc, "moe_gather_sum")
+    return out
+
+
+def moe_combine_bwd(g, y, w, pos, token_of=None):
     if y.dtype not in N._FLOATS or g.dtype != y.dtype or not g.is_contiguous() or pos.dtype != torch.int32:
         return NotImplemented
     T, k = w.shape
     cols = y.shape[1]
-    dy = torch.zeros_like(y)
+    # with the sort's row -> token table only the rows without a token are zeroed, by the kernel
+    pads = (token_of is not None and token_of.dtype == torch.int32 and token_of.is_contiguous()
+            and token_of.numel() == y.shape[0] and cols * y.element_size() % 16 == 0
+            and g.data_ptr() % 16 == 0 and y.data_ptr() % 16 == 0)
+    dy = torch.empty_like(y) if pads else torch.zeros_like(y)
     dw = torch.empty(T, k, dtype=torch.float32, device=y.device)
-    N._chk(N.lib().gb_moe_combine_bwd(g.data_ptr(), y.data_ptr(), w.contiguous().data_ptr(),
-                                      pos.contiguous().data_ptr(), dy.data_ptr(), dw.data_ptr(), T, k, cols,
-                                      N._DT[y.dtype], N._st()), "moe_combine_bwd")
+    w, pos = w.contiguous(), pos.contiguous()
+    N._chk(N.lib().gb_moe_combine_bwd(g.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(),
+                                      token_of.data_ptr() if pads else None, dy.data_ptr(), dw.data_ptr(), T,
+                                      y.shape[0], k, cols, N._DT[y.dtype], N._st()), "moe_combine_bwd")
     return dy, dw

@@ -45,7 +45,7 @@ _SIGS = {
     "gb_opt_chunk": "", "gb_adam_multi": "pilfffffffiipppp", "gb_adam_dyn_advance": "pddpp", "gb_copy_h2d_async": "pplp", "gb_sgd_multi": "pilfffp",
     "gb_grad_multi": "pilpfppip",
     "gb_router_fwd": "ppppp" + "liiiip", "gb_router_bwd": "pppppp" + "liiiip",
-    "gb_moe_sort": "pppppp" + "liiilp", "gb_moe_combine": "pppp" + "liiip", "gb_moe_combine_bwd": "pppppp" + "liiip",
+    "gb_moe_sort": "pppppp" + "liiilp", "gb_moe_combine": "pppp" + "liiip", "gb_moe_combine_bwd": "ppppppp" + "lliiip",
     "gb_gemm": "pppp" + "iiii" + "ll" + "i" + "lll" + "ii" + "iii" + "i" + "f" + "i" + "p" + "i" + "ii" + "p" + "i" + "p",
     "gb_gemm_pair": "ppppp" + "iii" + "ll" + "ii" + "ii" + "iii" + "i" + "f" + "ii" + "pp",
     "gb_allreduce_fused": "ppllii" + "I" + "f" + "p" + "i" + "p" + "ii" + "u" + "ppp",
@@ -1471,9 +1471,14 @@ def moe_combine(y, w, pos):
     return grouped.moe_combine(y, w, pos)
 
 
-def moe_combine_bwd(g, y, w, pos):
+def moe_gather_sum(y, pos):
     from . import grouped
-    return grouped.moe_combine_bwd(g, y, w, pos)
+    return grouped.moe_gather_sum(y, pos)
+
+
+def moe_combine_bwd(g, y, w, pos, token_of=None):
+    from . import grouped
+    return grouped.moe_combine_bwd(g, y, w, pos, token_of)
 
 
 # =============================== sort / select / index producers ================================
