@@ -33,8 +33,8 @@ _SIGS = {
     "gb_where": "pppffiiplip", "gb_cast": "ppliip", "gb_fill": "plfip", "gb_axpy": "ppfliip",
     "gb_copy_strided": "ppipppip", "gb_transpose": "ppiiilllip",
     "gb_reduce_rows": "ippllfiip", "gb_reduce_mid": "ipplllifiip",
-    "gb_rmsnorm_fwd": "pppplifiip", "gb_rmsnorm_bwd": "pppppplii" + "ip",
-    "gb_add_rmsnorm_fwd": "pppppplifiip", "gb_add_rmsnorm_bwd": "ppppppplii" + "ip", "gb_layernorm_fwd": "pppppplifiip",
+    "gb_rmsnorm_fwd": "pppplifiip", "gb_rmsnorm_bwd": "pppppplii" + "ipp",
+    "gb_add_rmsnorm_fwd": "pppppplifiipp", "gb_add_rmsnorm_bwd": "ppppppplii" + "ipp", "gb_layernorm_fwd": "pppppplifiip",
     "gb_layernorm_bwd": "pppppppp" + "liiip", "gb_norm_bwd_ctas": "l", "gb_rmsnorm_bwd_ctas": "lii",
     "gb_softmax_fwd_stream": "ppllii" + "pp", "gb_rmsnorm_fwd_stream": "pppplifii" + "pp", "gb_softmax_fwd": "ppllii" + "p", "gb_softmax_bwd": "pppllii" + "p",
     "gb_ce_fwd": "ppppllliip", "gb_ce_bwd": "ppppplll" + "iip",
@@ -837,8 +837,8 @@ def add_rmsnorm_fwd(x, res, w, eps):
     s, y = torch.empty_like(x), torch.empty_like(x)
     rstd = torch.empty(rows, dtype=F32, device=x.device)
     _chk(lib().gb_add_rmsnorm_fwd(x.data_ptr(), res.data_ptr(), s.data_ptr(), w.data_ptr(), y.data_ptr(),
-                                  rstd.data_ptr(), rows, cols, float(eps), _DT[x.dtype], _wdt(x, w), _st()),
-         "add_rmsnorm_fwd")
+                                  rstd.data_ptr(), rows, cols, float(eps), _DT[x.dtype], _wdt(x, w),
+                                  status_tensor(x.device).data_ptr(), _st()), "add_rmsnorm_fwd")
     return s, y, rstd
 
 
@@ -854,8 +854,8 @@ def add_rmsnorm_bwd(g, gres, x, w, rstd):
     dx = torch.empty_like(x)
     part = torch.empty(nct * cols, dtype=F32, device=x.device)
     _chk(L.gb_add_rmsnorm_bwd(g.data_ptr(), gres.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
-                              dx.data_ptr(), part.data_ptr(), rows, cols, _DT[x.dtype], _wdt(x, w), _st()),
-         "add_rmsnorm_bwd")
+                              dx.data_ptr(), part.data_ptr(), rows, cols, _DT[x.dtype], _wdt(x, w),
+                              status_tensor(x.device).data_ptr(), _st()), "add_rmsnorm_bwd")
     return dx, _colsum(part, nct, cols)
 
 
@@ -873,7 +873,8 @@ def rmsnorm_bwd(g, x, w, rstd):
     dx = torch.empty_like(x)
     part = torch.empty(nct * cols, dtype=F32, device=x.device)
     _chk(L.gb_rmsnorm_bwd(g.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), part.data_ptr(),
-                          rows, cols, _DT[x.dtype], _wdt(x, w), _st()), "rmsnorm_bwd")
+                          rows, cols, _DT[x.dtype], _wdt(x, w), status_tensor(x.device).data_ptr(), _st()),
+         "rmsnorm_bwd")
     return dx, _colsum(part, nct, cols)
 
 

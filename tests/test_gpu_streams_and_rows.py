@@ -22,6 +22,33 @@ def _rnd(*shape, dt=torch.float32, seed=0):
 ROUND = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}
 
 
+@pytest.mark.parametrize("rows,cols", [(1183, 1032), (1184, 1032), (1185, 1536), (1500, 2056), (1777, 4096), (1300, 8192),
+                                       (1200, 4104), (1184, 512)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+def test_wide_rmsnorm(rows, cols, dt):
+    x, res, g, gres = (_rnd(rows, cols, dt=dt, seed=i) for i in range(4))
+    w = _rnd(cols, seed=9)
+    s, y, rstd = N.add_rmsnorm_fwd(x, res, w, 1e-6)
+    N.check_status()
+    sd = (x.double() + res.double()).to(dt).double() if dt != torch.float32 else s.double()
+    assert torch.equal(s.double(), sd)
+    r = torch.rsqrt(sd.square().mean(-1, keepdim=True) + 1e-6)
+    ref = sd * r * w.double()
+    # one rounding of the result; the fp32 sum of `cols` squares is good to 2^-18
+    assert bool(((y.double() - ref).abs() <= (ROUND[dt] + 2.0 ** -18) * ref.abs() + 1e-7).all())
+    for extra in (None, gres):
+        dx, dw = N.rmsnorm_bwd(g, s, w, rstd) if extra is None else N.add_rmsnorm_bwd(g, extra, s, w, rstd)
+        N.check_status()
+        xh, gw = sd * r, g.double() * w.double()
+        want = r * (gw - xh * (gw * xh).mean(-1, keepdim=True)) + (0 if extra is None else extra.double())
+        size = r * gw.abs() + want.abs() + r * xh.abs()
+        assert bool(((dx.double() - want).abs() <= ROUND[dt] * want.abs() + 2.0 ** -17 * size + 1e-7).all())
+        dref = (g.double() * xh).sum(0)
+        assert float((dw.double() - dref).norm()) <= 1e-5 * float(dref.norm())
+        again = N.rmsnorm_bwd(g, s, w, rstd) if extra is None else N.add_rmsnorm_bwd(g, extra, s, w, rstd)
+        assert torch.equal(dx, again[0]) and torch.equal(dw, again[1])
+
+
 @pytest.mark.parametrize("T,k,E,cols", [(1, 1, 2, 8), (37, 2, 8, 136), (300, 8, 16, 2048), (129, 8, 128, 256), (64, 3, 5, 20)])
 def test_moe_row_sums(T, k, E, cols):
     g = torch.Generator(device=DEV).manual_seed(T)
