@@ -309,6 +309,53 @@ static int cast_from(const void* src, void* dst, long long n, int ddt, cudaStrea
   return (int)cudaGetLastError();
 }
 
+// Several fp32 tensors -> one 16-bit buffer, one after another (the parameters that a fused layer multiplies as one
+// matrix).  One launch instead of one per tensor: at 128 to 900 rows a conversion of its own takes less time on the GPU
+// than its launch does.  (24 layers, prefill of 2 x 333 tokens without kept 16-bit weights: 436 launches -> 316.)
+namespace gb {
+constexpr int CAST_STACK_MAX = 8;
+struct CastStack {
+  const float* src[CAST_STACK_MAX];
+  long long end[CAST_STACK_MAX];          // running total of 8-element units
+  int n;
+};
+template <typename TO>
+__global__ void cast_stack_kernel(const CastStack l, TO* __restrict__ out) {
+  const long long total = l.end[l.n - 1];
+  for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (long long)gridDim.x * blockDim.x) {
+    const float* src = l.src[0];
+    long long first = 0;
+#pragma unroll
+    for (int i = 1; i < CAST_STACK_MAX; ++i)
+      if (i < l.n && u >= l.end[i - 1]) { src = l.src[i]; first = l.end[i - 1]; }
+    const float4* p = reinterpret_cast<const float4*>(src + (u - first) * 8);
+    const float4 a = p[0], b = p[1];
+    Vec16<TO> o;
+    o.v[0] = Cvt<TO>::from_f(a.x); o.v[1] = Cvt<TO>::from_f(a.y); o.v[2] = Cvt<TO>::from_f(a.z); o.v[3] = Cvt<TO>::from_f(a.w);
+    o.v[4] = Cvt<TO>::from_f(b.x); o.v[5] = Cvt<TO>::from_f(b.y); o.v[6] = Cvt<TO>::from_f(b.z); o.v[7] = Cvt<TO>::from_f(b.w);
+    st16(out + u * 8, o);
+  }
+}
+}  // namespace gb
+
+// src[i]: 16-byte aligned, numel[i] > 0 elements, a multiple of 8; out_dt: DT_BF16 or DT_F16
+extern "C" int gb_cast_stack(const long long* src, const long long* numel, int n, void* out, int out_dt, cudaStream_t st) {
+  if (n < 1 || n > CAST_STACK_MAX) return -2;
+  CastStack l{};
+  l.n = n;
+  long long units = 0;
+  for (int i = 0; i < n; ++i) {
+    if (numel[i] <= 0 || numel[i] % 8 != 0) return -3;
+    l.src[i] = reinterpret_cast<const float*>(src[i]);
+    l.end[i] = units += numel[i] / 8;
+  }
+  const int grid = gb_grid(units, 256);
+  if (out_dt == DT_BF16) cast_stack_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(l, (__nv_bfloat16*)out);
+  else if (out_dt == DT_F16) cast_stack_kernel<__half><<<grid, 256, 0, st>>>(l, (__half*)out);
+  else return -2;
+  return (int)cudaGetLastError();
+}
+
 extern "C" int gb_cast(const void* src, void* dst, long long n, int sdt, int ddt, cudaStream_t st) {
   if (n == 0) return 0;
   if (sdt == DT_F32) return cast_from<float>(src, dst, n, ddt, st);

@@ -1532,12 +1532,7 @@ def _fused_params(tensors, dtype):
     hit = amp_state.cache.get(key)
     if hit is not None and all(a is b for a, b in zip(hit[0], tensors)):
         return hit[1]
-    rows = builtins.sum(t.shape[0] for t in tensors)
-    out = torch.empty((rows,) + tuple(tensors[0].shape[1:]), dtype=dtype, device=tensors[0].device)
-    o = 0
-    for t in tensors:
-        K.copy_(out[o:o + t.shape[0]], t)
-        o += t.shape[0]
+    out = K.cat_cast(tensors, dtype)
     if amp_state.enabled:
         amp_state.cache[key] = (list(tensors), out)
     return out

@@ -99,6 +99,19 @@ def copy_(dst, src):
     return dst
 
 
+def cat_cast(tensors, dtype):
+    """torch.cat(tensors) along dim 0, in `dtype`."""
+    rows = sum(t.shape[0] for t in tensors)
+    out = torch.empty((rows,) + tuple(tensors[0].shape[1:]), dtype=dtype, device=tensors[0].device)
+    if out.is_cuda and len(tensors) > 1 and N.cast_stack(tensors, out) is not NotImplemented:
+        return out
+    o = 0
+    for t in tensors:
+        copy_(out[o:o + t.shape[0]], t)
+        o += t.shape[0]
+    return out
+
+
 def contiguous(t):
     if t.is_contiguous():
         return t

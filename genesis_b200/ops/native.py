@@ -66,6 +66,7 @@ _SIGS = {
     "gb_scatter_dim": "ppp" + "d" + "ii" + "ii" + "pppp" + "l" + "ii" + "pp",
     "gb_index_get": "pp" + "ppp" + "i" + "pp",
     "gb_index_put": "pp" + "d" + "ii" + "ppp" + "i" + "pp",
+    "gb_cast_stack": "ppipip",
     "gb_masked_fill": "pp" + "d" + "ll" + "i" + "p", "gb_fill_elems": "pldip",
 }
 
@@ -314,6 +315,23 @@ def cast(t, dtype):
         return NotImplemented
     out = torch.empty(t.shape, dtype=dtype, device=t.device)
     _chk(lib().gb_cast(t.data_ptr(), out.data_ptr(), t.numel(), _DT[t.dtype], _DT[dtype], _st()), "cast")
+    return out
+
+
+def cast_stack(tensors, out):
+    """Up to eight fp32 tensors converted into the 16-bit `out`, one after another, by one launch."""
+    n = len(tensors)
+    if n > 8 or out.dtype not in (torch.bfloat16, torch.float16) or not out.is_contiguous() or out.data_ptr() % 16:
+        return NotImplemented
+    src, num = [], []
+    for t in tensors:
+        p, k = t.data_ptr(), t.numel()
+        if t.dtype != F32 or not t.is_contiguous() or p % 16 or k % 8 or k == 0:
+            return NotImplemented
+        src.append(p)
+        num.append(k)
+    _chk(lib().gb_cast_stack((ctypes.c_longlong * n)(*src), (ctypes.c_longlong * n)(*num), n, out.data_ptr(),
+                             _DT[out.dtype], _st()), "cast_stack")
     return out
 
 

@@ -68,3 +68,16 @@ def test_moe_row_sums(T, k, E, cols):
         assert bool(((dy.double() - want).abs() <= 2.0 ** -8 * want.abs()).all())
         dref = (rows * gr.double()[:, None]).sum(-1)
         assert bool(((dw.double() - dref).abs() <= 1e-4 * cols ** 0.5).all())
+
+
+@pytest.mark.parametrize("shapes", [[(896, 896), (128, 896), (128, 896)], [(8,), (16,)], [(5, 24)] * 8, [(3, 5), (4, 5)],
+                                    [(2, 8)] * 9, [(40000, 64), (1, 64)]])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_stacked_conversion(shapes, dt):
+    ts = [_rnd(*s, seed=i) for i, s in enumerate(shapes)]
+    assert torch.equal(K.cat_cast(ts, dt), torch.cat(ts).to(dt))
+    # the same from a base that is not 16-byte aligned, and from parameters that already have the dtype
+    un = [_rnd(t.numel() + 1)[1:].reshape(t.shape) for t in ts]
+    assert torch.equal(K.cat_cast(un, dt), torch.cat(un).to(dt))
+    low = [t.to(dt) for t in ts]
+    assert torch.equal(K.cat_cast(low, dt), torch.cat(low))
