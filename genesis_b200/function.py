@@ -20,6 +20,7 @@ import torch
 
 from . import grad_mode
 from .amp_state import amp_state, shadow_of
+from .tensor import Tensor
 
 
 # GENESIS_NVTX=1: one NVTX range per Function forward (and "<name>.backward" per backward node), for timelines
@@ -90,7 +91,6 @@ class Function:
 
     @classmethod
     def apply(cls, *args, **kwargs):
-        from .tensor import Tensor
         policy = cls.amp_policy
         st = amp_state
         # ---- AMP casting / promotion --------------------------------------------
@@ -104,16 +104,26 @@ class Function:
         elif policy is not AMPPolicy.PRESERVE:
             args = _promote_args(args)
 
-        # ---- collect tensor inputs ----------------------------------------------
+        # ---- collect tensor inputs (and, for built-in functions, the plain tensors behind them) -------------------
         grad_on = grad_mode.is_grad_enabled()
-        tensor_inputs = []
+        raw = cls.raw
+        tensor_inputs, raw_args = [], []
         for a in args:
             if isinstance(a, Tensor):
                 tensor_inputs.append(a)
+                raw_args.append(a._t)
             elif isinstance(a, (list, tuple)) and a and isinstance(a[0], Tensor):
                 tensor_inputs.extend(a)
-        needs = tuple(t.requires_grad for t in tensor_inputs) if grad_on else (False,) * len(tensor_inputs)
-        track = any(needs)
+                if raw:
+                    raw_args.append(type(a)(x._t for x in a))
+            else:
+                raw_args.append(a)
+        track = False
+        if grad_on:
+            needs = tuple([t.requires_grad for t in tensor_inputs])
+            track = any(needs)
+        else:
+            needs = (False,) * len(tensor_inputs)
 
         node = cls.__new__(cls)
         ctx = Context()
@@ -125,8 +135,7 @@ class Function:
         if _NVTX:
             torch.cuda.nvtx.range_push(cls.__name__)
         try:
-            if cls.raw:
-                raw_args = tuple(_unwrap(a) for a in args)
+            if raw:
                 out = cls.forward(ctx, *raw_args, **kwargs)
             else:
                 out = cls.forward(ctx, *args, **kwargs)
@@ -161,17 +170,7 @@ class Function:
         return tuple(results) if is_tuple else results[0]
 
 
-def _unwrap(a):
-    from .tensor import Tensor
-    if isinstance(a, Tensor):
-        return a._t
-    if isinstance(a, (list, tuple)) and a and isinstance(a[0], Tensor):
-        return type(a)(x._t for x in a)
-    return a
-
-
 def _autocast_args(args, dtype):
-    from .tensor import Tensor
     out = None
     for i, a in enumerate(args):
         if isinstance(a, Tensor):
@@ -190,7 +189,6 @@ def _autocast_args(args, dtype):
 
 def _promote_args(args):
     """Mixed float32 + float16/bfloat16 inputs are computed in float32."""
-    from .tensor import Tensor
     has32 = haslow = False
     for a in args:
         if isinstance(a, Tensor):
@@ -278,7 +276,6 @@ def cast_to_bf16(a):
 def check_dtype(value, dtype):
     """True when `value` (a tensor, or dicts / lists / tuples of them) contains a tensor of `dtype`
     (reference `function.py:130-147`)."""
-    from .tensor import Tensor
     if isinstance(value, Tensor):
         return value.dtype == dtype
     if isinstance(value, dict):

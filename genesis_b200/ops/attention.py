@@ -32,26 +32,30 @@ def _lib():
 
 
 def _supported(q, k, v):
-    if q.dtype not in (torch.bfloat16, torch.float16) or k.dtype != q.dtype or v.dtype != q.dtype:
+    dt, qs, ks = q.dtype, q.shape, k.shape
+    if (dt is not torch.bfloat16 and dt is not torch.float16) or k.dtype is not dt or v.dtype is not dt:
         return False
-    if q.dim() != 4 or k.dim() != 4 or k.shape != v.shape:
+    if len(qs) != 4 or len(ks) != 4 or ks != v.shape:
         return False
-    B, S, Hq, D = q.shape
-    if D not in (64, 128) or k.shape[0] != B or k.shape[3] != D or Hq % k.shape[2] or k.shape[1] < S or S == 0:
+    B, S, Hq, D = qs
+    Bk, Sk, Hkv, Dk = ks
+    if D not in (64, 128) or Bk != B or Dk != D or Hq % Hkv or Sk < S or S == 0:
         return False
-    return all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (q, k, v))
+    return (q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0)
 
 
 def forward(q, k, v, causal, scale):
     if not _supported(q, k, v):
         return NotImplemented
     B, S, Hq, D = q.shape
-    Sk, Hkv = k.shape[1], k.shape[2]
+    _, Sk, Hkv, _ = k.shape
+    dev = q.device
     o = torch.empty_like(q)
-    lse = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
+    lse = torch.empty(B, Hq, S, dtype=torch.float32, device=dev)
     N._chk(_lib().gb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, S, Sk, Hq,
-                              Hkv, D, 1 if causal else 0, float(scale), 1 if q.dtype == torch.bfloat16 else 0,
-                              N.status_tensor(q.device).data_ptr(), N._st()), "attn_fwd")
+                              Hkv, D, 1 if causal else 0, float(scale), 1 if q.dtype is torch.bfloat16 else 0,
+                              N.status_tensor(dev).data_ptr(), N._st()), "attn_fwd")
     return o, lse
 
 

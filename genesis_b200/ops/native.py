@@ -91,7 +91,8 @@ available = _lib.available
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of the current device's current stream, without the Stream object around it: read on every launch
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 launch_count = 0   # native launches since import (every wrapper call below launches >= 1 kernel)
