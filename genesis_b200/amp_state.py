@@ -64,14 +64,27 @@ def stacked_shadow_of(raws, dtype):
 # address of a low-precision weight copy [N, K] (or of a group's stacked buffer) -> its transposed twin [K, N], kept
 # current by the same optimizer step that refreshes the copy.  The data-gradient GEMM of a linear layer reads the twin
 # so that both of its operands are contiguous along the contraction (the layout the tensor cores read fastest).
+# An entry names its copy by a weak reference besides the address: it leaves with the copy (an optimizer that was
+# collected), and another tensor that later gets the same address does not find the twin of the old one.
 transposed = {}
+
+
+def keep_transposed(lp, twin):
+    key = lp.data_ptr()
+
+    def gone(ref):
+        e = transposed.get(key)
+        if e is not None and e[0] is ref:
+            del transposed[key]
+    transposed[key] = (weakref.ref(lp, gone), twin)
 
 
 def transposed_of(lp):
     """The [K, N] twin of the low-precision weight `lp` [N, K] when the optimizer maintains one, else None."""
     if not transposed:
         return None
-    t = transposed.get(lp.data_ptr())
+    e = transposed.get(lp.data_ptr())
+    t = e[1] if e is not None and e[0]() is lp else None
     if t is None or t.dtype != lp.dtype or t.dim() != 2 or lp.dim() != 2 or t.shape[0] != lp.shape[1] \
             or t.shape[1] != lp.shape[0]:
         return None

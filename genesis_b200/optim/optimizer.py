@@ -181,7 +181,7 @@ class _AdamBase(Optimizer):
         return self
 
     def _add_transposed(self, lp):
-        from ..amp_state import transposed as registry
+        from ..amp_state import keep_transposed
         twin = torch.empty(lp.shape[1], lp.shape[0], dtype=lp.dtype, device=lp.device)
         if lp.is_cuda:
             if K.transpose_into(twin, lp) is NotImplemented:
@@ -189,7 +189,7 @@ class _AdamBase(Optimizer):
         else:
             twin.copy_(lp.t())
         self._transposed.append((lp, twin))
-        registry[lp.data_ptr()] = twin
+        keep_transposed(lp, twin)
 
     def _refresh_transposed(self):
         for lp, twin in getattr(self, "_transposed", ()):
