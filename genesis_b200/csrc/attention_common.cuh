@@ -63,6 +63,23 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// 2^x for x <= 127 on the FMA pipes, two at a time: x is split into its nearest integer (the low bits of x + 1.5 * 2^23,
+// offset by the exponent bias so that a shift turns them into the scale) and a rest in [-1/2, 1/2], whose power is a
+// polynomial of degree 5, a least-squares fit on Chebyshev nodes reweighted until its relative error was level: 7.5e-8 in
+// exact arithmetic, 2^-22.2 in fp32, as good as ex2.approx.  Below 2^-126 the result stays at 2^-126; NaN passes through.
+__device__ __forceinline__ float2 poly_exp2(float2 x) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-126.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-126.f));
+  constexpr float MAGIC = 12582912.f + 127.f;
+  const float2 u = add2(x, make_float2(MAGIC, MAGIC));
+  const float2 f = fma2(add2(u, make_float2(-MAGIC, -MAGIC)), make_float2(-1.f, -1.f), x);
+  float2 p = fma2(f, make_float2(1.327647129e-3f, 1.327647129e-3f), make_float2(9.675540961e-3f, 9.675540961e-3f));
+  p = fma2(p, f, make_float2(5.550713092e-2f, 5.550713092e-2f));
+  p = fma2(p, f, make_float2(2.402212024e-1f, 2.402212024e-1f));
+  p = fma2(p, f, make_float2(6.931469440e-1f, 6.931469440e-1f));
+  p = fma2(p, f, make_float2(1.0000001192f, 1.0000001192f));
+  return mul2(p, make_float2(__uint_as_float(__float_as_uint(u.x) << 23), __uint_as_float(__float_as_uint(u.y) << 23)));
+}
 
 // ------------------------------------------------------------------------------------------------
 // host
