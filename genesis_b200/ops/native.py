@@ -581,25 +581,69 @@ def _plan(M, N, K, es, can_split, sms):
     return bn, 1
 
 
+def _k_parts(M, N, K, sms):
+    """Into how many equal parts the contraction of a 16-bit product with a 16-bit result is cut when its 128 x 256 tiles
+    leave much of the GPU idle and the contraction is long (the data gradient of the vocabulary projection, a down
+    projection of few tokens): the parts are the batches of one launch with fp32 results, which a reduction then adds up
+    in a fixed order.  1 = not at all.  The estimate is 5 ns per contraction element and wave of tiles, against the
+    traffic of the partial results (written and read in fp32, at 2 TB/s: the stores of a short wave overlap with nothing)
+    and one more launch.  Measured, whole against parts, us: 16 x 896 x 151936 566 / 69 (16 parts), 512 x 896 x 151936
+    570 / 135 (8), 1024 573 / 254 (4), 2048 638 / 506 (2), 50 x 896 x 32000 145 / 27 (16), 1211 x 1536 x 32000 130 / 114 (2),
+    666 x 1536 x 8960 42 / 32 (4); not at 3000 x 896 x 151936 (833 / 724 with one layout, 864 / 905 with the other), and not
+    below K = 8192, where launches are what is left (16 x 896 x 4864 25.7 / 27.6 and 25.3 / 22.8)."""
+    tiles = -(-M // 128) * -(-N // 256)
+    if K < 8192 or tiles > sms or K % 8 or N % 4:
+        return 1
+    best, parts = 0.8 * K * 5e-3, 1                              # microseconds; a split has to promise a fifth
+    for s in (2, 3, 4, 6, 8, 12, 16):
+        if K % (8 * s):
+            continue
+        t = -(-tiles * s // sms) * (K // s) * 5e-3 + 8 * s * M * N / 2e6 + 8
+        if t < best:
+            best, parts = t, s
+    return parts
+
+
+def _gemm_k_parts(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, s, out_dtype, alpha, sms):
+    kp = K // s
+    part = torch.empty(s, M, N, dtype=F32, device=a2.device)
+    _chk(lib().gb_gemm(a2.data_ptr(), b2.data_ptr(), part.data_ptr(), None, M, N, kp, s, lda, ldb, N,
+                       kp * lda if a_mn else kp, kp * ldb if b_mn else kp, M * N, a_mn, b_mn, _GEMM_DT[a2.dtype],
+                       _GEMM_DT[F32], 0, 0, float(alpha), 0, None, 0, 1, 0, status_tensor(a2.device).data_ptr(), sms,
+                       _st()), "gemm")
+    return _reduce3(0, part, 1, s, M * N, 1.0, out_dtype).view(M, N)
+
+
 pair_mode = os.environ.get("GENESIS_GEMM_PAIR", "auto")     # "auto" | "0" (never) | "1" (whenever the kernel applies)
 
 
-def _pair_width(M, N, K, sms, a_mn=0, b_mn=0):
-    """256 when the CTA-pair kernel (256 x 256 tiles on SM pairs) is expected to beat the single-CTA kernel for this
-    problem, else 0.  Measured on the model's shapes: the pair kernel wins by 2-9 % on K-major x K-major products with
-    many tiles and a short contraction (the forward projections out of the hidden size, where operand traffic into
-    the SMs bounds the 128 x 256 tile: +7 % at 16384 x 4864 x 896 and 16384 x 1152 x 896), loses on long contractions
-    (-2 % at K = 4864, -4 % at 16384 x 2048 x 8192, -15 % at 16384 cubed, where the single-CTA kernel's grouped
-    rasterisation keeps more of both operands in L2), on MN-major operands (data / weight gradients) and on very wide
-    outputs (the vocabulary projection); narrower pair tiles never pay."""
+def _pairs_win(M, N, sms, bn):
+    """Whether the CTA-pair kernel (256 x 256 tiles on SM pairs) is expected to beat whole tiles of the single-CTA kernel
+    (128 rows by `bn` columns).  A pair reads 64 KB of operands per 64-wide k step and two single CTAs 96 KB, so a full
+    wave of pairs takes 0.87 of the time of a full wave of 128 x 256 tiles (a wave of 128 x 128 tiles 0.6); what speaks
+    against pairs is a last wave that is nearly empty.  Measured, pair against single, us: 8192 x 151936 x 896 1610 / 2106,
+    16384 x 4864 x 896 108 / 124, 16384 x 896 x 4864 127 / 140, 4096 cubed 101 / 117, 16384 cubed 6382 / 7018, 1024 x 4864 x
+    896 25 / 29; with MN-major operands 16384 x 4864 x 896 114 / 139, 16384 x 1536 x 17920 657 / 699, 1536 x 8960 x 16384
+    347 / 383; where the rule says no: 2048 x 896 x 896 18.4 / 15.7, 896 x 4864 x 16384 238 / 125."""
+    single = -(-(-(-M // 128) * -(-N // bn)) // sms) * (1.0 if bn == 256 else 0.6)
+    return -(-(-(-M // 256) * -(-N // 256)) // (sms // 2)) * 0.87 < single
+
+
+def _pair_width(M, N, K, sms, a_mn=0, b_mn=0, bn=256):
+    """Tile width of the CTA-pair kernel for a product of two K-major operands, 0 where the single-CTA kernel (tiles
+    `bn` wide) takes it."""
     if pair_mode == "0":
         return 0
     if pair_mode == "1":
         return 256
-    if a_mn or b_mn or M < 2048 or N < 768 or N > 32768 or K > 1536:
-        return 0
-    tiles = -(-M // 256) * -(-N // 256)
-    return 256 if tiles >= 2 * (sms // 2) else 0
+    return 256 if not (a_mn or b_mn) and _pairs_win(M, N, sms, bn) else 0
+
+
+def _pair_width_mn(M, N, sms, bn):
+    """The same where an operand is MN-major."""
+    if pair_mode != "auto":
+        return 256 if pair_mode == "1" else 0
+    return 256 if _pairs_win(M, N, sms, bn) else 0
 
 
 def gemm_pair(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, out, bias, accumulate, alpha, bn):
@@ -698,7 +742,7 @@ def gemm(a, b_t, out_dtype=None, bias=None, accum=None, alpha=1.0, out=None):
     if plan_override is not None:
         bn, splits = plan_override
     elif splits == 1 and a.element_size() == 2:
-        pbn = _pair_width(M, N, K, sms, a_mn, b_mn)
+        pbn = _pair_width_mn(M, N, sms, bn) if a_mn or b_mn else _pair_width(M, N, K, sms, bn=bn)
         if pbn and gemm_pair(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, out, bias, accum is not None, alpha, pbn):
             return out
     if splits < 0 and (out.data_ptr() % 16 or (N * out.element_size()) % 16):
