@@ -718,6 +718,12 @@ def gemm(a, b_t, out_dtype=None, bias=None, accum=None, alpha=1.0, out=None):
     out_dtype = out_dtype or a.dtype
     if out_dtype not in _GEMM_DT:
         return NotImplemented
+    if K >= 8192 and M and N and accum is None and out is None and bias is None and out_dtype != F32 and a.dtype != F32 \
+            and plan_override is None:
+        sms = _sms(a.device)
+        s = _k_parts(M, N, K, sms)
+        if s > 1:
+            return _gemm_k_parts(*_operand(a, True), *_operand(b_t, True), M, N, K, s, out_dtype, alpha, sms)
     if accum is not None:
         out = accum
         if not out.is_contiguous():

@@ -81,3 +81,18 @@ def test_stacked_conversion(shapes, dt):
     assert torch.equal(K.cat_cast(un, dt), torch.cat(un).to(dt))
     low = [t.to(dt) for t in ts]
     assert torch.equal(K.cat_cast(low, dt), torch.cat(low))
+
+
+@pytest.mark.parametrize("M,Nc,K", [(1, 8, 8192), (5, 64, 8192), (130, 264, 8960), (300, 896, 8192), (129, 40, 32000),
+                                   (2048, 896, 30016), (64, 512, 8200)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_long_contractions(M, Nc, K, dt):
+    """Products whose contraction may be cut into parts, in the layouts of a forward pass and of a data gradient."""
+    a, b = _rnd(M, K, dt=dt), _rnd(Nc, K, dt=dt, seed=1)
+    ref, size = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    for got in (lambda: N.gemm(a, b), lambda: N.linear_dgrad(a, b.t().contiguous()), lambda: N.gemm(a.t().contiguous().t(), b)):
+        out = got()
+        N.check_status()
+        # one rounding of the result; fp32 accumulation of K products in runs of 16: K / 16 roundings of 2^-24
+        assert bool(((out.double() - ref).abs() <= ROUND[dt] * ref.abs() + K / 16 * 2.0 ** -24 * size + 1e-7).all())
+        assert torch.equal(out, got())
