@@ -1,6 +1,6 @@
 """Row kernels at the edges of their routes: RMSNorm rows that stream through the ring (row lengths from the first past
-the warp-per-row kernel to the longest, row counts around the ring's turn), the mixture-of-experts row sums, stacked
-parameter conversions, and products with a long contraction."""
+the warp-per-row kernel to the longest, row counts around the ring's turn), cross-entropy rows, the mixture-of-experts row
+sums, stacked parameter conversions, and products with a long contraction."""
 import pytest
 import torch
 
@@ -47,6 +47,25 @@ def test_wide_rmsnorm(rows, cols, dt):
         assert float((dw.double() - dref).norm()) <= 1e-5 * float(dref.norm())
         again = N.rmsnorm_bwd(g, s, w, rstd) if extra is None else N.add_rmsnorm_bwd(g, extra, s, w, rstd)
         assert torch.equal(dx, again[0]) and torch.equal(dw, again[1])
+
+
+@pytest.mark.parametrize("cols", [8, 1000, 4096, 4096 + 8, 8192 - 8, 32771, 151936])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+def test_cross_entropy_rows(cols, dt):
+    x = _rnd(6, cols, dt=dt) * 4
+    x[1] = -float("inf")                     # one finite entry among masked ones, at the end of the row
+    x[1, -1] = 2.0
+    x[2, 0] = 60.0                           # the maximum comes first
+    x[3] = torch.finfo(dt).min               # all of them the lowest value
+    x[5, cols // 2] = float("nan")
+    t = torch.tensor([0, cols - 1, 0, cols // 2, -100, 0], device=DEV)
+    loss, lse = N.cross_entropy_fwd(x, t, -100)
+    ref = torch.logsumexp(x.double(), -1)
+    # fp32 exponentials and sums of up to 151936 terms in runs of some hundreds: a few 2^-20 of a value of about 10
+    assert bool(((lse.double() - ref).abs()[:5] <= 1e-5 * ref.abs()[:5].clamp_min(1)).all()) and bool(lse[5].isnan())
+    pick = x.double()[torch.arange(6), t.clamp_min(0)]
+    assert bool(((loss.double() - (ref - pick)).abs()[:4] <= 1e-5 * (ref.abs() + pick.abs())[:4].clamp_min(1)).all())
+    assert float(loss[4]) == 0.0
 
 
 @pytest.mark.parametrize("T,k,E,cols", [(1, 1, 2, 8), (37, 2, 8, 136), (300, 8, 16, 2048), (129, 8, 128, 256), (64, 3, 5, 20)])
