@@ -320,17 +320,22 @@ def cast(t, dtype):
 
 
 def cast_stack(tensors, out):
-    """Up to eight fp32 tensors converted into the 16-bit `out`, one after another, by one launch."""
+    """Up to eight fp32 tensors converted into the 16-bit `out`, one after another along dim 0, by one launch.  All have
+    to lie on the device of `out`, and their rows have to be those of `out`: the caller's copies, one by one, take (or
+    refuse) anything else."""
     n = len(tensors)
     if n > 8 or out.dtype not in (torch.bfloat16, torch.float16) or not out.is_contiguous() or out.data_ptr() % 16:
         return NotImplemented
     src, num = [], []
+    dev, row = out.device, out.shape[1:]
     for t in tensors:
         p, k = t.data_ptr(), t.numel()
-        if t.dtype != F32 or not t.is_contiguous() or p % 16 or k % 8 or k == 0:
+        if t.dtype != F32 or t.device != dev or t.shape[1:] != row or not t.is_contiguous() or p % 16 or k % 8 or k == 0:
             return NotImplemented
         src.append(p)
         num.append(k)
+    if sum(num) != out.numel():
+        return NotImplemented
     _chk(lib().gb_cast_stack((ctypes.c_longlong * n)(*src), (ctypes.c_longlong * n)(*num), n, out.data_ptr(),
                              _DT[out.dtype], _st()), "cast_stack")
     return out

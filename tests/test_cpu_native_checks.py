@@ -1,0 +1,41 @@
+"""What the wrappers of the native kernels look at before they pass an address on: an operand on another device, or one
+that the kernel's wide loads could not read, never reaches a launch.  The native library is replaced by a recorder."""
+import pytest
+import torch
+
+import genesis_b200  # noqa: F401
+from genesis_b200.ops import dispatch as K
+from genesis_b200.ops import native as N
+
+
+class _Recorder:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append(name)
+            return 0
+        return call
+
+
+@pytest.fixture
+def native(monkeypatch):
+    rec = _Recorder()
+    monkeypatch.setattr(N, "lib", lambda: rec)
+    monkeypatch.setattr(N, "_st", lambda: 0)
+    monkeypatch.setattr(N, "status_tensor", lambda dev: torch.zeros(8, dtype=torch.int32))
+    return rec
+
+
+def test_stacked_conversion_takes_one_device_and_whole_rows(native):
+    a, b = torch.randn(4, 8), torch.randn(2, 8)
+    out = torch.empty(6, 8, dtype=torch.bfloat16)
+    assert N.cast_stack([a, b], out) is out and native.calls == ["gb_cast_stack"]
+    native.calls.clear()
+    for ts in ([a, b.to("meta")], [a.to("meta"), b], [a, torch.randn(4, 4)], [a, torch.randn(16)], [a, torch.randn(1, 8)]):
+        assert N.cast_stack(ts, out) is NotImplemented
+    assert native.calls == []
+    # rows that do not match are refused by the copies, as a concatenation would
+    with pytest.raises(RuntimeError):
+        K.cat_cast([a, torch.randn(4, 4)], torch.bfloat16)
