@@ -1126,10 +1126,16 @@ def _token_rows(t):
     return rs, True
 
 
+def _tables_ok(dev, cos, sin, positions):
+    """Rotation tables (and positions) that a kernel on `dev` can read: one left on the host, by a module that was not
+    moved, is torch's to take or to refuse."""
+    return (cos.dtype == F32 and sin.dtype == F32 and cos.device == dev and sin.device == dev and cos.is_contiguous()
+            and sin.is_contiguous() and (positions is None or positions.device == dev))
+
+
 def rope(x, cos, sin, positions, inverse, out=None):
     """Rotate-half RoPE.  `x` and `out` may be column slices of wider matrices (equal token-row spacing)."""
-    if x.dtype not in _FLOATS or x.dim() != 4 or cos.dtype != F32 or sin.dtype != F32 \
-            or not cos.is_contiguous() or not sin.is_contiguous() or x.shape[-1] % 2:
+    if x.dtype not in _FLOATS or x.dim() != 4 or x.shape[-1] % 2 or not _tables_ok(x.device, cos, sin, positions):
         return NotImplemented
     xrs, ok = _token_rows(x)
     if not ok:
@@ -1158,8 +1164,7 @@ def qkv_rope(y, q, k, v, cos, sin, positions, Hq, Hkv, D, merge):
     rotated q, rotated k, v, all freshly allocated when passed as None) or merge (`merge=True`: gradients q, k, v ->
     y, rotated back).  Returns (y, q, k, v) or NotImplemented."""
     t = y if y is not None else q
-    if t.dtype not in _FLOATS or cos.dtype != F32 or sin.dtype != F32 or not cos.is_contiguous() \
-            or not sin.is_contiguous():
+    if t.dtype not in _FLOATS or not _tables_ok(t.device, cos, sin, positions):
         return NotImplemented
     B, S = t.shape[0], t.shape[1]
     Nt = (Hq + 2 * Hkv) * D

@@ -39,3 +39,21 @@ def test_stacked_conversion_takes_one_device_and_whole_rows(native):
     # rows that do not match are refused by the copies, as a concatenation would
     with pytest.raises(RuntimeError):
         K.cat_cast([a, torch.randn(4, 4)], torch.bfloat16)
+
+
+@pytest.mark.parametrize("away", ["cos", "sin", "positions"])
+def test_rotation_tables_of_another_device(native, away):
+    B, S, Hq, Hkv, D = 2, 5, 2, 1, 8
+    t = {"cos": torch.randn(16, D), "sin": torch.randn(16, D), "positions": torch.arange(S)}
+    y, q, kv = torch.randn(B, S, (Hq + 2 * Hkv) * D), torch.randn(B, S, Hq, D), torch.randn(B, S, Hkv, D)
+
+    def launches():
+        native.calls.clear()
+        r = (N.rope(q, t["cos"], t["sin"], t["positions"], False),
+             N.qkv_rope(y, None, None, None, t["cos"], t["sin"], t["positions"], Hq, Hkv, D, False),
+             N.qkv_rope(None, q, kv, kv, t["cos"], t["sin"], t["positions"], Hq, Hkv, D, True))
+        return [x is NotImplemented for x in r], len(native.calls)
+
+    assert launches() == ([False] * 3, 3)
+    t[away] = t[away].to("meta")
+    assert launches() == ([True] * 3, 0)
