@@ -876,6 +876,11 @@ def _norm_ok(x, cols):
         and cols // v <= 256 * 8
 
 
+def _weights_ok(x, w, cols):
+    """Weights (or biases) that the row kernels can read in 16-byte pieces: one per column, on the device of x."""
+    return w.numel() == cols and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.device == x.device
+
+
 def _wdt(x, w):
     if w.dtype == F32 or w.dtype == x.dtype:
         return _DT[w.dtype]
@@ -884,7 +889,7 @@ def _wdt(x, w):
 
 def rmsnorm_fwd(x, w, eps):
     cols = x.shape[-1]
-    if not _norm_ok(x, cols) or _wdt(x, w) is None or not w.is_contiguous():
+    if not _norm_ok(x, cols) or _wdt(x, w) is None or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     y = torch.empty_like(x)
@@ -905,7 +910,7 @@ def add_rmsnorm_fwd(x, res, w, eps):
     """(s = x + res, rmsnorm(s) * w, rstd) in one pass over the rows."""
     cols = x.shape[-1]
     if not _norm_ok(x, cols) or not _norm_ok(res, cols) or res.dtype != x.dtype or res.shape != x.shape \
-            or _wdt(x, w) is None or not w.is_contiguous():
+            or _wdt(x, w) is None or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     s, y = torch.empty_like(x), torch.empty_like(x)
@@ -920,7 +925,7 @@ def add_rmsnorm_bwd(g, gres, x, w, rstd):
     """(rmsnorm_backward(g) + gres, dw): the gradient of either addend of the sum that was normalised."""
     cols = x.shape[-1]
     if not _norm_ok(x, cols) or not _norm_ok(g, cols) or not _norm_ok(gres, cols) or g.dtype != x.dtype \
-            or gres.dtype != x.dtype or _wdt(x, w) is None:
+            or gres.dtype != x.dtype or _wdt(x, w) is None or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     L = lib()
@@ -939,7 +944,8 @@ def _colsum(partial, nrows, cols):
 
 def rmsnorm_bwd(g, x, w, rstd):
     cols = x.shape[-1]
-    if not _norm_ok(x, cols) or not _norm_ok(g, cols) or g.dtype != x.dtype or _wdt(x, w) is None:
+    if not _norm_ok(x, cols) or not _norm_ok(g, cols) or g.dtype != x.dtype or _wdt(x, w) is None \
+            or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     L = lib()
@@ -958,7 +964,8 @@ def layernorm_fwd(x, w, b, eps):
         return NotImplemented
     ref = w if w is not None else b
     wdt = _DT[x.dtype] if ref is None else _wdt(x, ref)
-    if wdt is None or (w is not None and b is not None and w.dtype != b.dtype):
+    if wdt is None or (w is not None and b is not None and w.dtype != b.dtype) \
+            or any(t is not None and not _weights_ok(x, t, cols) for t in (w, b)):
         return NotImplemented
     rows = x.numel() // cols
     y = torch.empty_like(x)
@@ -975,7 +982,7 @@ def layernorm_bwd(g, x, w, mean, rstd):
     if not _norm_ok(x, cols) or not _norm_ok(g, cols) or g.dtype != x.dtype:
         return NotImplemented
     wdt = _DT[x.dtype] if w is None else _wdt(x, w)
-    if wdt is None:
+    if wdt is None or (w is not None and not _weights_ok(x, w, cols)):
         return NotImplemented
     rows = x.numel() // cols
     L = lib()

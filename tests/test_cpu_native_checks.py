@@ -57,3 +57,25 @@ def test_rotation_tables_of_another_device(native, away):
     assert launches() == ([False] * 3, 3)
     t[away] = t[away].to("meta")
     assert launches() == ([True] * 3, 0)
+
+
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+def test_norm_weights_that_the_kernels_cannot_read(native, monkeypatch, wdt):
+    monkeypatch.setattr(N, "_colsum", lambda *a: None)
+    rows, cols = 3, 16
+    x, rstd = torch.randn(rows, cols).bfloat16(), torch.ones(rows)
+    monkeypatch.setattr(_Recorder, "gb_rmsnorm_bwd_ctas", lambda *a: 1, raising=False)
+    monkeypatch.setattr(_Recorder, "gb_norm_bwd_ctas", lambda *a: 1, raising=False)
+
+    def refused(w):
+        native.calls.clear()
+        r = (N.rmsnorm_fwd(x, w, 1e-6), N.add_rmsnorm_fwd(x, x, w, 1e-6), N.rmsnorm_bwd(x, x, w, rstd),
+             N.add_rmsnorm_bwd(x, x, x, w, rstd), N.layernorm_fwd(x, w, None, 1e-6), N.layernorm_fwd(x, None, w, 1e-6),
+             N.layernorm_bwd(x, x, w, rstd, rstd))
+        return {y is NotImplemented for y in r}, len(native.calls)
+
+    base = torch.ones(2 * cols + 8, dtype=wdt)
+    assert base.data_ptr() % 16 == 0
+    assert refused(base[:cols]) == ({False}, 7)
+    for w in (base[1:cols + 1], base[:2 * cols:2], base[:cols].to("meta"), base[:cols - 1], base[:1]):
+        assert refused(w) == ({True}, 0)
