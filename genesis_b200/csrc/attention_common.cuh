@@ -65,11 +65,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
 
 // 2^x for x <= 127 on the FMA pipes, two at a time: x is split into its nearest integer (the low bits of x + 1.5 * 2^23,
 // offset by the exponent bias so that a shift turns them into the scale) and a rest in [-1/2, 1/2], whose power is a
-// polynomial of degree 5, a least-squares fit on Chebyshev nodes reweighted until its relative error was level: 7.5e-8 in
-// exact arithmetic, 2^-22.2 in fp32, as good as ex2.approx.  Below 2^-126 the result stays at 2^-126; NaN passes through.
+// polynomial of degree 5, a least-squares fit on Chebyshev nodes reweighted until its relative error was level: 1.55e-7 in
+// exact arithmetic with the constants as rounded here, 2^-22.1 in fp32, as good as ex2.approx.  At -127 the scale's exponent
+// bits are all zero, so everything from -126.5 down, -inf included, becomes exactly 0 (ex2.approx.ftz: from -126 down); a
+// clamp one higher would leave 2^-126 there, and a row whose scores are all -inf would come out as the mean of V.  NaN
+// passes through.
 __device__ __forceinline__ float2 poly_exp2(float2 x) {
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-126.f));
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-126.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-127.f));
   constexpr float MAGIC = 12582912.f + 127.f;
   const float2 u = add2(x, make_float2(MAGIC, MAGIC));
   const float2 f = fma2(add2(u, make_float2(-MAGIC, -MAGIC)), make_float2(-1.f, -1.f), x);

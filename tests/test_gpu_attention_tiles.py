@@ -79,6 +79,33 @@ def test_forward_with_growing_scores(shape, ramp):
     _check_fwd(*_inputs(*shape, torch.bfloat16, ramp=ramp), True)
 
 
+@pytest.mark.parametrize("S,Sk", [(1, 512), (200, 512), (300, 1000)])       # decoding, unmasked tiles only, a ragged last tile
+@pytest.mark.parametrize("D", [64, 128])
+def test_forward_with_scores_of_minus_infinity(S, Sk, D):
+    """Overflowed products: a row whose scores are all -inf is empty (output 0, lse -inf) on every route; in the other rows a
+    key whose score is -inf has probability exactly 0, whatever its value."""
+    q, k, v = _inputs(2, S, Sk, 4, 2, D, torch.bfloat16)
+    q[..., 0], k[..., 0] = 0.0, -1e30
+    q[0, S // 2, :, :], k[0, :Sk // 3, 0, 1], v[0, :Sk // 3, 0] = 0.0, -1e30, 3e38
+    q[0, S // 2, :, 0] = 1e30                        # 1e30 * -1e30: all scores of this row
+    q[..., 1] = q[..., 1].abs() + 1e10               # 1e10 * -1e30: the first third of its keys, for the first group
+    q[0, S // 2, :, 1] = 0.0
+    k[0, Sk // 3:, 0, 1] = k[1, :, :, 1] = k[:, :, 1, 1] = 0.0
+    r = N.attention_fwd(q, k, v, False, D ** -0.5)
+    N.check_status()
+    o, lse = r
+    assert bool((o[0, S // 2] == 0).all()) and bool((lse[0, :, S // 2] == -math.inf).all())
+    if S > 1:
+        live = torch.ones(S, dtype=torch.bool, device=DEV)
+        live[S // 2] = False
+        vz = v.clone()
+        vz[0, :Sk // 3, 0] = 0                       # what 0 * v leaves
+        ref, lref, pv = _oracle(q, k, vz, False, D ** -0.5)
+        bound = (2.0 ** -8 + 2.0 ** -16) * (pv + ref.abs()) + 1e-6          # as in _check_fwd
+        assert bool(((o.double() - ref).abs() <= bound)[:, live].all())
+        assert float((lse.double() - lref)[..., live].abs().max()) <= 2e-5 * float(lref[..., live].abs().max())
+
+
 BWD = [
     (1, 127, 127, 2, 1, 64), (1, 129, 130, 4, 2, 128), (2, 256, 256, 6, 3, 64), (1, 385, 500, 14, 2, 64),
     (1, 40, 700, 4, 1, 128), (4, 520, 520, 12, 2, 128), (8, 650, 650, 14, 2, 64), (2, 384, 384, 5, 5, 128),
