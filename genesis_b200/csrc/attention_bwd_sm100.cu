@@ -118,13 +118,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
       mbar_expect_tx(qdo_full, 2 * TILE);
       load_tile<D>(sQ, &tmq, qdo_full, h, m0, b, AT_BM);
       load_tile<D>(sdO, &tmdo, qdo_full, h, m0, b, AT_BM);
-      for (int j = 0; j < n_kv; ++j) {
+      int j = 0;
+      for (; j < n_kv; ++j) {
         const int st = j % ST;
         if (!AT_WAIT(&kv_empty[st], ((j / ST) & 1) ^ 1, 40)) break;
         mbar_expect_tx(&kv_full[st], 2 * TILE);
         load_tile<D>(sKV + st * 2 * TILE, &tmk, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
         load_tile<D>(sKV + st * 2 * TILE + TILE, &tmv, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
       }
+      if (*abort_flag) { drain_copies(qdo_full, 1, 1); drain_copies(kv_full, ST, j); }
     }
   } else if (warp == 9) {
     // ---------------- MMA: the warp stays converged, one elected lane issues ----------------
@@ -314,8 +316,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
       load_tile<D>(sK, &tmk, kv_full, kvh, n0, b, AT_BM);
       load_tile<D>(sV, &tmv, kv_full, kvh, n0, b, AT_BM);
       const size_t half = (size_t)p.B * p.Hq * p.Spad;
-      int h = h0, qt = i_start;
-      for (int it = 0; it < n_it; ++it) {
+      int h = h0, qt = i_start, it = 0;
+      for (; it < n_it; ++it) {
         const int st = it % ST;
         if (!AT_WAIT(&q_empty[st], ((it / ST) & 1) ^ 1, 60)) break;
         mbar_expect_tx(&q_full[st], STAGE + C::STATS);
@@ -326,6 +328,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
         bulk_load(sStat + st * C::STATS + AT_BM * 4, src + half, AT_BM * 4, &q_full[st]);
         if (++qt == nq) { qt = i_start; ++h; }
       }
+      if (*abort_flag) { drain_copies(kv_full, 1, 1); drain_copies(q_full, ST, it); }
     }
   } else if (warp == 9) {
     // ---------------- MMA: the warp stays converged, one elected lane issues ----------------

@@ -184,6 +184,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
     if (lane == 0 && c + DC_ST * DC_WARPS < c1) load(c + DC_ST * DC_WARPS, st);
   }
 
+  if (__any_sync(0xffffffffu, *abort_flag)) {      // gave up: this warp's last loads have to land first
+    const int mine = c1 > c0 ? (c1 - c0 + DC_WARPS - 1) / DC_WARPS : 0;
+    drain_copies(full, DC_ST, mine < it + DC_ST ? mine : it + DC_ST);
+    __syncwarp();
+  }
   // the warps' parts, in shared memory in the place of their rings (every load has arrived and been read)
   float* part = reinterpret_cast<float*>(ring);
 #pragma unroll

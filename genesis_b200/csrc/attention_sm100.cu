@@ -112,13 +112,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
   if (warp == 8) {
     if (lane == 0) {   // ---------------- TMA ----------------
       tma_prefetch_desc(&tmq); tma_prefetch_desc(&tmk); tma_prefetch_desc(&tmv); tma_prefetch_desc(&tmo);
-      int slot = 0, qn[2] = {0, 0};
+      int slot = 0;
       uint32_t par = 0;                       // parity of the ring's current lap
+      uint32_t qn[2] = {0, 0}, kvn = 0;       // loads issued
       bool ok = true;
       auto load_kv = [&](const CUtensorMap* m, int head, int row, int b) {
         if (!ok || !(ok = AT_WAIT(&kv_empty[slot], par ^ 1, 10))) return;
         mbar_expect_tx(&kv_full[slot], TILE);
         load_tile<D>(sKV + slot * TILE, m, &kv_full[slot], head, row, b, AT_BN);
+        ++kvn;
         if (++slot == ST) { slot = 0; par ^= 1; }
       };
       for (int r = 0; ok && r < rounds; ++r) {
@@ -138,6 +140,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__
           load_kv(&tmv, kvh, j * AT_BN, w.b);
           if (j + 1 < w.nmax) load_kv(&tmk, kvh, (j + 1) * AT_BN, w.b);
         }
+      }
+      if (*abort_flag) {
+        drain_copies(kv_full, ST, kvn);
+        drain_copies(&q_full[0], 1, qn[0]);
+        drain_copies(&q_full[1], 1, qn[1]);
       }
     }
   } else if (warp == 9) {

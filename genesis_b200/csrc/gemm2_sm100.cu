@@ -286,14 +286,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ 
         }
         if (!ok) { give_up(); break; }
       }
-      if (*abort_flag && rank == 0) {
-        // give loads in flight a bounded time to land before shared memory is given up
-        for (int s = 0; s < STAGES; ++s) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(&full_bar[s], 0) && !mbar_try_wait(&full_bar[s], 1) &&
-                 globaltimer_ns() - t0 < 1000000ull) {}
-        }
-      }
+      // (the leader's barriers count the loads of both CTAs, which meet once more before they leave)
+      if (*abort_flag && rank == 0) drain_copies(full_bar, STAGES, it);
     }
     __syncwarp();
   } else if (warp == 1) {

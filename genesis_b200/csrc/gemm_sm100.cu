@@ -221,15 +221,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ C
           }
         }
       }
-      // Drain: every load issued above has been (or will be) consumed by the MMA warp, which
-      // waits on the full barriers; on abort, give in-flight copies a bounded time to land.
-      if (*abort_flag) {
-        for (int s = 0; s < STAGES; ++s) {
-          uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(&full_bar[s], 0) && !mbar_try_wait(&full_bar[s], 1) &&
-                 globaltimer_ns() - t0 < 1000000ull) {}
-        }
-      }
+      // every load issued above has been (or will be) consumed by the MMA warp, which waits on the full barriers,
+      // unless a role gave up
+      if (*abort_flag) drain_copies(full_bar, STAGES, it);
     }
   } else if (warp == 1) {
     // ====== MMA issuer: the warp stays converged (its addresses live in uniform registers), one elected lane issues ======

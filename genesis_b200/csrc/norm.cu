@@ -196,6 +196,11 @@ struct NormRing {
     bulk_load(dst + row_bytes, (const uint8_t*)b + row * row_bytes, row_bytes, &full[st]);
     if (parts == 3) bulk_load(dst + 2 * (size_t)row_bytes, (const uint8_t*)c + row * row_bytes, row_bytes, &full[st]);
   }
+  // rows row, row + grid, ... have been asked for, as many as there are stages
+  __device__ __forceinline__ void drain(long long row, long long rows) const {
+    const uint32_t done = (uint32_t)(row / gridDim.x), mine = (uint32_t)((rows - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    drain_copies(full, stages, done + stages < mine ? done + stages : mine);
+  }
 };
 
 // s = x + res (rounded to T), y = s * rstd(s) * w
@@ -231,7 +236,10 @@ add_rmsnorm_fwd_stream_kernel(const T* __restrict__ x, const T* __restrict__ res
   int st = 0;
   uint32_t ph = 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
-    if (!mbar_wait(&full[st], ph, &abort_flag, status, 710)) break;
+    if (!mbar_wait(&full[st], ph, &abort_flag, status, 710)) {
+      if (threadIdx.x == 0) ring.drain(row, rows);
+      break;
+    }
     const T* a = reinterpret_cast<const T*>(ns_smem + (size_t)st * 2 * ring.row_bytes);
     const T* b = a + cols;
     Vec16<T> buf[NV];
@@ -306,7 +314,10 @@ rmsnorm_bwd_stream_kernel(const T* __restrict__ g, const T* __restrict__ x, cons
   uint32_t ph = 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const float r = rstd[row];
-    if (!mbar_wait(&full[st], ph, &abort_flag, status, 711)) break;
+    if (!mbar_wait(&full[st], ph, &abort_flag, status, 711)) {
+      if (threadIdx.x == 0) ring.drain(row, rows);
+      break;
+    }
     const T* a = reinterpret_cast<const T*>(ns_smem + (size_t)st * parts * ring.row_bytes);
     Vec16<T> xb[NV], gb_[NV], gr[NV];
     float dot = 0.f;

@@ -49,9 +49,9 @@ row_stream_kernel(const T* __restrict__ x, long long rows, int cols, Op op, int*
     const uint32_t ph = (it >> 1) & 1;
     const bool ok = mbar_wait(&full[s], ph, &abort_flag, status, 700);
     if (!__syncthreads_and(ok ? 1 : 0)) {
-      // a copy that never arrived: the other stage may still be in flight; give it its own bounded wait so that
-      // nothing is written into this CTA's shared memory after it has left
-      if (threadIdx.x == 0 && r + stride < rows) mbar_wait(&full[s ^ 1], (uint32_t)(((it + 1) >> 1) & 1), &abort_flag, nullptr, 701);
+      // a copy that never arrived: those still in flight may not be written into shared memory that this CTA has left
+      const long long mine = (rows - blockIdx.x + stride - 1) / stride;
+      if (threadIdx.x == 0) drain_copies(full, 2, (uint32_t)(it + 2 < mine ? it + 2 : mine));
       return;
     }
     op.row(state, reinterpret_cast<const T*>(rs_smem + (size_t)s * row_bytes), r, cols, sh);

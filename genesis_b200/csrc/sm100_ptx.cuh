@@ -108,6 +108,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Before a role that gave up leaves: the copies that it has issued get a millisecond to land, so that none is written into
+// the shared memory of the CTA that comes next.  Copy number i went to stage i % stages and completes phase i / stages of
+// full[i % stages].  (Asking for both parities instead would ask for nothing: one of them is always over.)
+__device__ __forceinline__ void drain_copies(uint64_t* full, uint32_t stages, uint32_t issued) {
+  const uint64_t t0 = globaltimer_ns();
+  for (uint32_t i = issued > stages ? issued - stages : 0; i < issued; ++i)
+    while (!mbar_try_wait(&full[i % stages], (i / stages) & 1) && globaltimer_ns() - t0 < 1000000ull) {}
+}
+
 // ---------------------------------------------------------------------------------------------
 // fences
 // ---------------------------------------------------------------------------------------------

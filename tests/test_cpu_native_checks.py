@@ -1,5 +1,8 @@
 """What the wrappers of the native kernels look at before they pass an address on: an operand on another device, or one
 that the kernel's wide loads could not read, never reaches a launch.  The native library is replaced by a recorder."""
+import os
+import re
+
 import pytest
 import torch
 
@@ -79,3 +82,27 @@ def test_norm_weights_that_the_kernels_cannot_read(native, monkeypatch, wdt):
     assert refused(base[:cols]) == ({False}, 7)
     for w in (base[1:cols + 1], base[:2 * cols:2], base[:cols].to("meta"), base[:cols - 1], base[:1]):
         assert refused(w) == ({True}, 0)
+
+
+def _kernels():
+    """(file, head, body) of every kernel in the sources."""
+    d = os.path.join(os.path.dirname(genesis_b200.__file__), "csrc")
+    for f in sorted(os.listdir(d)):
+        if f.endswith((".cu", ".cuh")):
+            src = open(os.path.join(d, f)).read()
+            for part in src.split("__global__ ")[1:]:
+                body = part[:part.index("\n}")]
+                yield f, " ".join(body[:120].split()), body
+
+
+def test_kernels_that_give_up_wait_for_their_copies():
+    """A kernel whose copies complete on barriers (its waits are bounded) lets the copies in flight land before it leaves.
+    The path cannot be provoked by a sound kernel, so this looks at the sources."""
+    seen = 0
+    for f, name, body in _kernels():
+        if "mbar_expect_tx(" in body or "ring.issue(" in body:
+            seen += 1
+            assert "drain_copies(" in body or "ring.drain(" in body, (f, name)
+        # a barrier is always past one of its two parities, so a wait for either of them ends at once
+        assert not re.search(r"!mbar_try_wait\(&?([^,]+), 0\) && !mbar_try_wait\(&?\1, 1\)", body), (f, name)
+    assert seen >= 9
