@@ -193,7 +193,7 @@ __global__ void softmax_bwd_kernel(const T* __restrict__ g, const T* __restrict_
   }
 }
 
-// The pass over a 16-bit row for the cross-entropy of a large vocabulary: two vectors in flight per thread, the maximum
+// The pass over a 16-bit row (16-byte aligned, whole vectors) for the cross-entropy of a large vocabulary: two vectors in flight per thread, the maximum
 // of their eight pairs taken in the 16-bit type (exact), differences, scaling and sums two at a time.  The scalar pass
 // issued six instructions per element and had one 16-byte load per thread in flight: [2048, 151936] bf16 166 -> 122 us
 // (5.1 TB/s).  512 threads, three CTAs on an SM, so that one row's barriers are under another's loads; four vectors per
@@ -248,26 +248,55 @@ __device__ __forceinline__ MaxSum row_maxsum16(const T* p, int cols, float* sh) 
   int i = threadIdx.x;
   for (; i + (int)blockDim.x < nv; i += 2 * blockDim.x) take(v[i], v[i + blockDim.x], true);
   if (i < nv) { const uint4 a = v[i]; take(a, a, false); }
-  for (int c = nv * 8 + threadIdx.x; c < cols; c += blockDim.x) {
-    const float x = Cvt<T>::to_f(p[c]);
-    if (x > acc.m) { acc.s *= __expf(acc.m - x); acc.m = x; }
-    if (acc.m != -INFINITY) acc.s += __expf(x - acc.m);
-  }
   return block_maxsum(acc, sh);
 }
 
 template <typename T, typename TI>
-__global__ void __launch_bounds__(sizeof(T) == 2 ? 512 : 1024, sizeof(T) == 2 ? 3 : 1)
+__global__ void __launch_bounds__(1024)
 ce_fwd_kernel(const T* __restrict__ logits, const TI* __restrict__ target, float* __restrict__ loss,
               float* __restrict__ lse_out, long long rows, long long cols, long long ignore_index) {
   __shared__ float sh[64];
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* p = logits + row * cols;
-    MaxSum ms;
-    if constexpr (sizeof(T) == 2)
-      ms = (cols < (1ll << 31) && (reinterpret_cast<uintptr_t>(p) & 15) == 0) ? row_maxsum16(p, (int)cols, sh) : row_maxsum(p, cols, sh);
-    else
-      ms = row_maxsum(p, cols, sh);
+    const MaxSum ms = row_maxsum(p, cols, sh);
+    if (threadIdx.x == 0) {
+      const float lse = ms.m + logf(ms.s);
+      lse_out[row] = lse;
+      const long long t = (long long)target[row];
+      loss[row] = (t == ignore_index || t < 0 || t >= cols) ? 0.f : lse - Cvt<T>::to_f(p[t]);
+    }
+  }
+}
+
+// The same with one CTA on an SM, whose threads may use 64 registers instead of 32: several loads per thread are in flight,
+// which pays on long aligned fp32 rows ([1024, 128256]: 112 -> 103 us; [64, 151936]: 18.4 -> 14.4) and nowhere else, for
+// then the barriers of a row are under no other row's loads ([2048, 8192] 33 -> 41, unaligned [2048, 50257] 191 -> 314).
+template <typename TI>
+__global__ void __launch_bounds__(1024, 1)
+ce_fwd_long_kernel(const float* __restrict__ logits, const TI* __restrict__ target, float* __restrict__ loss,
+                   float* __restrict__ lse_out, long long rows, long long cols, long long ignore_index) {
+  __shared__ float sh[64];
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    const float* p = logits + row * cols;
+    const MaxSum ms = row_maxsum(p, cols, sh);
+    if (threadIdx.x == 0) {
+      const float lse = ms.m + logf(ms.s);
+      lse_out[row] = lse;
+      const long long t = (long long)target[row];
+      loss[row] = (t == ignore_index || t < 0 || t >= cols) ? 0.f : lse - p[t];
+    }
+  }
+}
+
+// 16-byte aligned rows of a 16-bit type through the packed pass
+template <typename T, typename TI>
+__global__ void __launch_bounds__(512, 3)
+ce_fwd16_kernel(const T* __restrict__ logits, const TI* __restrict__ target, float* __restrict__ loss,
+                float* __restrict__ lse_out, long long rows, int cols, long long ignore_index) {
+  __shared__ float sh[64];
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    const T* p = logits + row * cols;
+    const MaxSum ms = row_maxsum16(p, cols, sh);
     if (threadIdx.x == 0) {
       const float lse = ms.m + logf(ms.s);
       lse_out[row] = lse;
@@ -543,15 +572,33 @@ extern "C" int gb_softmax_bwd(const void* g, const void* y, void* dx, long long 
   return (int)cudaGetLastError();
 }
 
+// The packed pass wants rows that are all aligned, and more than one vector per thread of them.  bf16, scalar pass / packed
+// pass, us: [4096, 2048] 24.6 / 26.6, [4096, 4096] 29.3 / 30.9, [4096, 4104] 33.1 / 34.7, [4096, 5120] 34.6 / 30.8,
+// [2048, 8192] 30.8 / 18.5, [2048, 151936] 158 / 107.
+template <typename T, typename TI>
+static void launch_ce_fwd(const void* logits, const void* target, float* loss, float* lse, long long rows, long long cols,
+                          long long ignore_index, int grid, cudaStream_t st) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && cols * sizeof(T) % 16 == 0;
+  if constexpr (sizeof(T) == 2) {
+    if (aligned && cols >= 5120 && cols < (1ll << 31)) {
+      ce_fwd16_kernel<T, TI><<<grid, 512, 0, st>>>((const T*)logits, (const TI*)target, loss, lse, rows, (int)cols, ignore_index);
+      return;
+    }
+  } else if (aligned && cols >= 65536) {
+    ce_fwd_long_kernel<TI><<<grid, 1024, 0, st>>>((const T*)logits, (const TI*)target, loss, lse, rows, cols, ignore_index);
+    return;
+  }
+  ce_fwd_kernel<T, TI><<<grid, row_block(cols), 0, st>>>((const T*)logits, (const TI*)target, loss, lse, rows, cols, ignore_index);
+}
+
 extern "C" int gb_ce_fwd(const void* logits, const void* target, float* loss, float* lse, long long rows,
                          long long cols, long long ignore_index, int dt, int target_is_i64, cudaStream_t st) {
   if (rows == 0) return 0;
   const int grid = (int)(rows < 148 * 8 ? rows : 148 * 8);
-  const int block = dt == DT_F32 ? row_block(cols) : (row_block(cols) < 512 ? row_block(cols) : 512);
   if (target_is_i64) {
-    GB_DISPATCH_FLOAT(dt, T, ce_fwd_kernel<T, long long><<<grid, block, 0, st>>>((const T*)logits, (const long long*)target, loss, lse, rows, cols, ignore_index));
+    GB_DISPATCH_FLOAT(dt, T, (launch_ce_fwd<T, long long>(logits, target, loss, lse, rows, cols, ignore_index, grid, st)));
   } else {
-    GB_DISPATCH_FLOAT(dt, T, ce_fwd_kernel<T, int><<<grid, block, 0, st>>>((const T*)logits, (const int*)target, loss, lse, rows, cols, ignore_index));
+    GB_DISPATCH_FLOAT(dt, T, (launch_ce_fwd<T, int>(logits, target, loss, lse, rows, cols, ignore_index, grid, st)));
   }
   return (int)cudaGetLastError();
 }
