@@ -178,9 +178,8 @@ rmsnorm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const TW* _
 // bulk copy) in shared memory.  The row-per-CTA kernels above load a row, meet at the barriers of its sum, store it, and
 // only then ask for the next one; here the copies of the next ST - 1 rows are in flight all the time.  The threads take a
 // row into registers before the barriers of its sum, so those barriers also tell that its stage can be filled again.
-// Weights (and, backward, the partial weight gradient) of a thread's columns stay in registers for all rows.
-// [8192, 4096] bf16, row-per-CTA kernels -> these: add + norm forward 55.4 -> 45.4 us (5.9 TB/s), backward with the
-// residual gradient 66.7 -> 46.0 us (5.8 TB/s).
+// Weights (and, backward, the partial weight gradient) of a thread's columns stay in registers for all rows.  Where the line
+// to the row-per-CTA kernels lies: norm_stream_stages.
 // ------------------------------------------------------------------------------------------
 constexpr int NS_SMEM = 108 * 1024;         // ring of one CTA: two CTAs on an SM
 constexpr int NS_MAX_NV = 4;                // 16-byte vectors of a row per thread
@@ -366,12 +365,32 @@ rmsnorm_bwd_stream_kernel(const T* __restrict__ g, const T* __restrict__ x, cons
   }
 }
 
-// Rows that the warp-per-row kernels do not take, enough of them for the ring to turn over on every CTA, and at least two
-// of them in it.
-static inline int norm_stream_stages(long long rows, int cols, int dt, int parts) {
-  const long long rb = (long long)cols * (dt == DT_F32 ? 4 : 2);
-  if (rb <= 2048 || rb > 16 * NORM_THREADS * NS_MAX_NV || rows < 4 * 296) return 0;
-  if (parts == 3 && cols > NS_MAX_BWD_COLS) return 0;
+static inline int norm_stream_ctas() { return 2 * sm_count(); }
+
+// Stages of the ring for rows that stream (the warp-per-row kernels have taken the narrow ones), 0 for the row-per-CTA
+// kernels.  There has to be a turn of the ring for every CTA.  Up to 2048 16-bit columns a thread of the row-per-CTA kernels
+// holds one vector of each operand (32 registers forward, 48 backward) and other CTAs cover for the one at its barriers; with
+// two (40 and 80) too few of them are left.
+// Row-per-CTA / streamed, us, inputs cycled past L2 (backward: with the residual gradient unless noted):
+//   forward  bf16: [8192, 1536] 22.4 / 26.5, [8192, 2048] 26.7 / 27.5, [2048, 3584] 12.5 / 14.4, [4096, 2560] 22.2 / 18.8,
+//            [8192, 2560] 46.4 / 32.9, [8192, 4096] 57.8 / 52.1, [32768, 4096] 218 / 192; rows whose inputs stay below 18 MB
+//            each fit L2 together, and the ring's start is not made up for ([2048, 4096] from L2: 10.3 / 12.4)
+//   forward  fp32: no gain anywhere ([8192, 4096] 87.2 / 92.8): not streamed
+//   backward bf16: [2048, 2304] 29.5 / 24.7, [8192, 2560] 85.8 / 51.4, [8192, 4096] 101 / 60, [32768, 4096] 347 / 178; without
+//            the residual gradient 74.7 / 55.8 and 235 / 163 at the last two
+//   backward fp32: [8192, 4096] 142 / 92; with two vectors a thread (1280 columns and more) where the operands exceed L2, too:
+//            [8192, 1536] 60 / 47, [32768, 1536] 196 / 138, without the residual gradient 44 / 43 and 136 / 127
+//   backward, narrower rows: without the residual gradient the row-per-CTA kernel is the better one ([32768, 2048] bf16
+//            106 / 126), with it the worse one only at many rows ([32768, 1536] bf16 126 / 114).  Both calls take one route, so
+//            that their weight gradients are the same bits.
+static inline int norm_stream_stages(long long rows, int cols, int dt, bool bwd) {
+  const long long rb = (long long)cols * (dt == DT_F32 ? 4 : 2), parts = bwd ? 3 : 2;
+  if (rb > 16 * NORM_THREADS * NS_MAX_NV || rows < 4 * norm_stream_ctas()) return 0;
+  if (bwd) {
+    if (cols > NS_MAX_BWD_COLS || (cols <= 2048 && (dt != DT_F32 || cols < 1280 || rows * rb < 32000000))) return 0;
+  } else if (dt == DT_F32 || cols <= 2048 || rows * rb < 18000000) {
+    return 0;
+  }
   const long long st = NS_SMEM / (parts * rb);
   return st < 2 ? 0 : (int)(st > 8 ? 8 : st);
 }
@@ -720,11 +739,15 @@ static int rmsnorm_fwd_impl(const void* x, const void* w, void* y, float* rstd, 
 template <typename T, typename TW, int NV>
 static int launch_add_fwd_stream(const void* x, const void* res, const void* w, void* sum_out, void* y, float* rstd,
                                  long long rows, int cols, float eps, int stages, int* status, cudaStream_t st) {
-  static unsigned long long cfg = 0;
-  if (int e = smem_opt_in(add_rmsnorm_fwd_stream_kernel<T, TW, NV>, NS_SMEM, cfg)) return e;
-  add_rmsnorm_fwd_stream_kernel<T, TW, NV><<<296, NORM_THREADS, (size_t)stages * 2 * cols * sizeof(T), st>>>(
-      (const T*)x, (const T*)res, (const TW*)w, (T*)sum_out, (T*)y, rstd, rows, cols, eps, stages, status);
-  return (int)cudaGetLastError();
+  if constexpr (sizeof(T) != 2 || NV == 1) {
+    return -2;                                // (norm_stream_stages lets no such row through)
+  } else {
+    static unsigned long long cfg = 0;
+    if (int e = smem_opt_in(add_rmsnorm_fwd_stream_kernel<T, TW, NV>, NS_SMEM, cfg)) return e;
+    add_rmsnorm_fwd_stream_kernel<T, TW, NV><<<norm_stream_ctas(), NORM_THREADS, (size_t)stages * 2 * cols * sizeof(T), st>>>(
+        (const T*)x, (const T*)res, (const TW*)w, (T*)sum_out, (T*)y, rstd, rows, cols, eps, stages, status);
+    return (int)cudaGetLastError();
+  }
 }
 template <typename T, typename TW, int NV>
 static int launch_bwd_stream(const void* g, const void* x, const void* w, const float* rstd, void* dx, float* dw_partial,
@@ -734,7 +757,7 @@ static int launch_bwd_stream(const void* g, const void* x, const void* w, const 
   } else {
     static unsigned long long cfg = 0;
     if (int e = smem_opt_in(rmsnorm_bwd_stream_kernel<T, TW, NV>, NS_SMEM, cfg)) return e;
-    rmsnorm_bwd_stream_kernel<T, TW, NV><<<296, NORM_THREADS, (size_t)stages * 3 * cols * sizeof(T), st>>>(
+    rmsnorm_bwd_stream_kernel<T, TW, NV><<<norm_stream_ctas(), NORM_THREADS, (size_t)stages * 3 * cols * sizeof(T), st>>>(
         (const T*)g, (const T*)x, (const TW*)w, rstd, (T*)dx, dw_partial, rows, cols, (const T*)gres, stages, status);
     return (int)cudaGetLastError();
   }
@@ -758,7 +781,7 @@ static int rmsnorm_fwd_impl(const void* x, const void* w, void* y, float* rstd, 
   if (rows == 0) return 0;
   if (!norm_cols_ok(cols, dt)) return -2;
   if (res != nullptr) {
-    const int stages = norm_stream_stages(rows, cols, dt, 2);
+    const int stages = norm_stream_stages(rows, cols, dt, false);
     if (stages > 0)
       NORM_STREAM_DISPATCH(dt, wdt, cols, return (launch_add_fwd_stream<T, TW, NV>(x, res, w, sum_out, y, rstd, rows, cols, eps, stages, status, st)));
   }
@@ -921,7 +944,7 @@ extern "C" int gb_rmsnorm_bwd_ctas(long long rows, int cols, int dt) {
     const long long want = (rows + NORM_BWD_WARPS - 1) / NORM_BWD_WARPS;
     return (int)(want < 148 ? want : 148);
   }
-  if (norm_stream_stages(rows, cols, dt, 3) > 0) return 296;
+  if (norm_stream_stages(rows, cols, dt, true) > 0) return norm_stream_ctas();
   return gb_norm_bwd_ctas(rows);
 }
 
@@ -938,7 +961,7 @@ static int rmsnorm_bwd_impl(const void* g, const void* x, const void* w, const f
     else if (nvec <= 64) { NORM_DISPATCH_T(dt, wdt, return (launch_rmsnorm_bwd_warp<T, TW, 2>(g, x, w, rstd, dx, dw_partial, rows, cols, gres, grid, st))); }
     else { NORM_DISPATCH_T(dt, wdt, return (launch_rmsnorm_bwd_warp<T, TW, 4>(g, x, w, rstd, dx, dw_partial, rows, cols, gres, grid, st))); }
   }
-  const int stages = norm_stream_stages(rows, cols, dt, 3);
+  const int stages = norm_stream_stages(rows, cols, dt, true);
   if (stages > 0)
     NORM_STREAM_DISPATCH(dt, wdt, cols, return (launch_bwd_stream<T, TW, NV>(g, x, w, rstd, dx, dw_partial, rows, cols, gres, stages, status, st)));
   NORM_DISPATCH(dt, wdt, cols, rmsnorm_bwd_kernel<T, TW, MV><<<grid, NORM_THREADS, 0, st>>>(

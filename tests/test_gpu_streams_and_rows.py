@@ -1,5 +1,5 @@
-"""Row kernels at the edges of their routes: RMSNorm rows that stream through the ring (row lengths from the first past
-the warp-per-row kernel to the longest, row counts around the ring's turn), cross-entropy rows, the mixture-of-experts row
+"""Row kernels at the edges of their routes: RMSNorm rows on both sides of the line to the kernels that stream rows through a
+ring (row lengths, row counts and total sizes, which differ forward, backward and with the type), cross-entropy rows, the mixture-of-experts row
 sums, stacked parameter conversions, and products with a long contraction."""
 import pytest
 import torch
@@ -23,7 +23,8 @@ ROUND = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.
 
 
 @pytest.mark.parametrize("rows,cols", [(1183, 1032), (1184, 1032), (1185, 1536), (1500, 2056), (1777, 4096), (1300, 8192),
-                                       (1200, 4104), (1184, 512)])
+                                       (1200, 4104), (1184, 512), (2197, 4096), (2198, 4096), (1184, 2056), (6250, 1280),
+                                       (6249, 1280)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
 def test_wide_rmsnorm(rows, cols, dt):
     x, res, g, gres = (_rnd(rows, cols, dt=dt, seed=i) for i in range(4))
