@@ -622,33 +622,23 @@ def _gemm_k_parts(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, s, out_dtype, alpha, sm
 pair_mode = os.environ.get("GENESIS_GEMM_PAIR", "auto")     # "auto" | "0" (never) | "1" (whenever the kernel applies)
 
 
-def _pairs_win(M, N, sms, bn):
-    """Whether the CTA-pair kernel (256 x 256 tiles on SM pairs) is expected to beat whole tiles of the single-CTA kernel
-    (128 rows by `bn` columns).  A pair reads 64 KB of operands per 64-wide k step and two single CTAs 96 KB, so a full
-    wave of pairs takes 0.87 of the time of a full wave of 128 x 256 tiles (a wave of 128 x 128 tiles 0.6); what speaks
-    against pairs is a last wave that is nearly empty.  Measured, pair against single, us: 8192 x 151936 x 896 1610 / 2106,
-    16384 x 4864 x 896 108 / 124, 16384 x 896 x 4864 127 / 140, 4096 cubed 101 / 117, 16384 cubed 6382 / 7018, 1024 x 4864 x
-    896 25 / 29; with MN-major operands 16384 x 4864 x 896 114 / 139, 16384 x 1536 x 17920 657 / 699, 1536 x 8960 x 16384
-    347 / 383; where the rule says no: 2048 x 896 x 896 18.4 / 15.7, 896 x 4864 x 16384 238 / 125."""
-    single = -(-(-(-M // 128) * -(-N // bn)) // sms) * (1.0 if bn == 256 else 0.6)
-    return -(-(-(-M // 256) * -(-N // 256)) // (sms // 2)) * 0.87 < single
-
-
-def _pair_width(M, N, K, sms, a_mn=0, b_mn=0, bn=256):
-    """Tile width of the CTA-pair kernel for a product of two K-major operands, 0 where the single-CTA kernel (tiles
-    `bn` wide) takes it."""
-    if pair_mode == "0":
-        return 0
-    if pair_mode == "1":
-        return 256
-    return 256 if not (a_mn or b_mn) and _pairs_win(M, N, sms, bn) else 0
-
-
-def _pair_width_mn(M, N, sms, bn):
-    """The same where an operand is MN-major."""
-    if pair_mode != "auto":
+def _pair_width(M, N, K, sms, bn):
+    """256 where the CTA-pair kernel (256 x 256 tiles on SM pairs) is expected to beat whole tiles of the single-CTA kernel
+    (128 rows by `bn` columns), else 0.  The layout of the operands makes no difference to the rule.
+    A pair reads 64 KB of operands per 64-wide k step and two single CTAs 96 KB, so a full wave of pairs takes 0.87 of the
+    time of a full wave of 128 x 256 tiles (a wave of 128 x 128 tiles 0.6); what speaks against pairs is a last wave that is
+    nearly empty, and their start (barriers across two CTAs), which costs as much as 48 elements of the contraction, or 128
+    where a single wave is all there is and nothing hides it.  Measured, us, single / pair, both operands K-major:
+    8192 x 32000 x 896 452 / 380, 4096 x 4864 x 896 36.6 / 32.9, 16384 cubed 7018 / 6382, 1024 x 4864 x 896 20.0 / 16.5, one
+    wave each: 256 x 18944 x 3584 35.6 / 32.8, 1024 x 3584 x 18944 121 / 108, 2048 x 1536 x 1536 15.9 / 16.5; with an MN-major
+    operand 4096 x 1536 x 1536 27.9 / 23.7; where the rule says no: 4096 x 896 x 896 12.4 / 13.6, 2048 x 896 x 896 10.3 / 12.4,
+    100 x 256 x 256 with an fp32 result 9.0 / 10.3, 896 x 4864 x 16384 125 / 238.  Over 956 products (M from 1 to 8192, N from
+    136 to 32000, K from 8 to 32000, three layouts) it is 0.2 % off the better of the two on average."""
+    if pair_mode in ("0", "1"):
         return 256 if pair_mode == "1" else 0
-    return 256 if _pairs_win(M, N, sms, bn) else 0
+    single = -(-(-(-M // 128) * -(-N // bn)) // sms)
+    pairs = -(-(-(-M // 256) * -(-N // 256)) // (sms // 2))
+    return 256 if pairs * 0.87 * K + (128 if single == 1 else 48) < single * (1.0 if bn == 256 else 0.6) * K else 0
 
 
 def gemm_pair(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, out, bias, accumulate, alpha, bn):
@@ -753,7 +743,7 @@ def gemm(a, b_t, out_dtype=None, bias=None, accum=None, alpha=1.0, out=None):
     if plan_override is not None:
         bn, splits = plan_override
     elif splits == 1 and a.element_size() == 2:
-        pbn = _pair_width_mn(M, N, sms, bn) if a_mn or b_mn else _pair_width(M, N, K, sms, bn=bn)
+        pbn = _pair_width(M, N, K, sms, bn)
         if pbn and gemm_pair(a2, a_mn, lda, b2, b_mn, ldb, M, N, K, out, bias, accum is not None, alpha, pbn):
             return out
     if splits < 0 and (out.data_ptr() % 16 or (N * out.element_size()) % 16):

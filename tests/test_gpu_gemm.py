@@ -211,14 +211,44 @@ def test_linear_swiglu_function_matches_the_unfused_layers():
     assert K.fallback_counts() == {}
 
 
-def test_gemm_routes_large_16_bit_shapes_to_the_pair_kernel():
+@pytest.mark.parametrize("M,Nc,K,pair", [
+    (4096, 4864, 896, True), (1024, 4864, 896, True),            # several waves, K-short: less operand traffic
+    (1000, 4872, 904, True),                                     # the same, ragged in every direction
+    (256, 4864, 4096, False), (2048, 896, 896, False),           # one nearly empty wave of pairs
+    (4096, 896, 896, False), (4096, 896, 1088, True),            # one wave of each: only where K hides the pair's start
+    (8, 136, 8, False), (129, 264, 72, False),
+])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+def test_gemm_routes_to_the_pair_kernel(monkeypatch, M, Nc, K, pair, a_mn, b_mn, out):
+    """Which products take CTA pairs, whatever the layout, and that they are right there; an fp32 result whose tiles leave
+    the last wave ragged goes to stream-K before the question arises."""
+    taken = []
+    real = N.gemm_pair
+    monkeypatch.setattr(N, "gemm_pair", lambda *a: taken.append(real(*a)) or taken[-1])
+    monkeypatch.setattr(N, "pair_mode", "auto")
+    ld = lambda t, mn: t.t().contiguous().t() if mn else t
+    a, b = rnd(M, K, dt=torch.bfloat16), rnd(Nc, K, dt=torch.bfloat16, seed=1)
     before = N.launch_count
-    a, b = rnd(4096, 896, dt=torch.bfloat16).to(DEV), rnd(4864, 896, dt=torch.bfloat16, seed=1).to(DEV)
-    assert N._pair_width(4096, 4864, 896, N._sms(a.device)) == 256
-    assert N._pair_width(4096, 4864, 896, N._sms(a.device), b_mn=1) == 0
-    got = N.gemm(a, b)
-    check(got, a.float().cpu() @ b.float().cpu().t(), torch.bfloat16, 896)
-    assert N.launch_count == before + 1
+    got = N.gemm(ld(a.to(DEV), a_mn), ld(b.to(DEV), b_mn), out_dtype=out)
+    ref = a.float() @ b.float().t()
+    check(got, ref, out, K)
+    sms = N._sms(got.device)
+    bn, splits = N._plan(M, Nc, K, 2, out == torch.float32, sms)
+    if splits == 1:
+        aligned = (M % 8 == 0 or not a_mn) and (Nc % 8 == 0 or not b_mn)
+        launched = bool(taken) and taken[-1]
+        if Nc * got.element_size() % 16 == 0:
+            assert launched == (N._pair_width(M, Nc, K, sms, bn) == 256)
+        if out == torch.bfloat16 and Nc % 8 == 0:
+            assert launched == pair
+            assert not aligned or N.launch_count == before + 1
+    else:
+        assert not taken
+    if out == torch.float32:
+        acc = got.clone()
+        N.gemm(ld(a.to(DEV), a_mn), ld(b.to(DEV), b_mn), out_dtype=out, accum=acc)
+        check(acc, 2 * ref, out, K)
 
 
 @pytest.mark.parametrize("M,I,H", [(256, 128, 64), (512, 256, 896), (1000, 448, 200), (2048, 4864, 896)])
