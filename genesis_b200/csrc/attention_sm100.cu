@@ -367,8 +367,11 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   if ((r = smem_opt_in(attn_fwd_kernel<D, BF16>, FwdCfg<D>::SMEM, cfg)) != 0) return r;
   const int sms = sm_count();
   const long long nq = (p.S + AT_BM - 1) / AT_BM, bh = (long long)p.B * p.Hq;
-  // two tiles per item once that still gives every SM an item of its own
-  const int tiles = ((nq + 1) / 2) * bh >= sms ? 2 : 1;
+  // Two tiles per item wherever that saves a round of the CTAs: two tiles in turn take little longer than one.  One tile / two
+  // tiles, us, d = 128, not causal: 24 heads, 1024 rows (2 rounds, 1) 35 / 23; 96 heads, 256 rows (2, 1) 16 / 12; 160 heads,
+  // 777 rows (8, 5) 111 / 79; as many rounds of pairs: 96 heads, 384 rows (2, 2) 18.6 / 22.2.  (660 shapes of 4 to 512 heads
+  // and 129 to 2048 rows: 0.3 % off the better of the two on average; pairs once they gave every SM an item: 2.7 %.)
+  const int tiles = (((nq + 1) / 2) * bh + sms - 1) / sms < (nq * bh + sms - 1) / sms ? 2 : 1;
   const long long items = ((nq + tiles - 1) / tiles) * bh;
   if (items > 0x7fffffff) return -5;
   attn_fwd_kernel<D, BF16><<<(int)(items < sms ? items : sms), FW_THREADS, FwdCfg<D>::SMEM, st>>>(tq, tk, tv, to, p,
