@@ -119,7 +119,9 @@ static inline int make_tmap_bshd(CUtensorMap* out, const void* base, int is_bf16
 
 
 
-// attention of a few query rows (attention_decode_sm100.cu); arguments as checked by gb_attn_fwd
+// attention of a few query rows (attention_decode_sm100.cu); arguments as checked by gb_attn_fwd.  decode_split: the CTAs that
+// share the keys of an item, and how many chunks of keys the longest warp then takes.
+void decode_split(const AttnParams& p, int D, int& ranks, int& steps);
 int attn_decode(const void* q, const void* k, const void* v, const AttnParams& p, int D, cudaStream_t st);
 
 }  // namespace gb

@@ -248,6 +248,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constan
   cluster.sync();          // nobody leaves while its shared memory is being read
 }
 
+// keys are split until two CTAs sit on every SM, as long as a warp keeps two chunks to itself; 8 is the portable limit
+void decode_split(const AttnParams& p, int D, int& ranks, int& steps) {
+  const int kc = D == 128 ? DecCfg<128>::KC : DecCfg<64>::KC;
+  const long long items = ((long long)p.S * (p.Hq / p.Hkv) + DC_ROWS - 1) / DC_ROWS * p.Hkv * p.B;
+  const int chunks = (p.Sk + kc - 1) / kc;
+  ranks = 1;
+  while (ranks < 8 && items * ranks < 2 * sm_count() && chunks >= 4 * ranks * DC_WARPS) ranks *= 2;
+  steps = (chunks + ranks * DC_WARPS - 1) / (ranks * DC_WARPS);
+}
+
 template <int D, bool BF16>
 static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const void* q, const AttnParams& p, cudaStream_t st) {
   using C = DecCfg<D>;
@@ -255,11 +265,8 @@ static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const voi
   int r;
   if ((r = smem_opt_in(attn_decode_kernel<D, BF16>, C::SMEM, cfg)) != 0) return r;
   const int tiles = (p.S * (p.Hq / p.Hkv) + DC_ROWS - 1) / DC_ROWS;
-  const long long items = (long long)tiles * p.Hkv * p.B;
-  const int chunks = (p.Sk + C::KC - 1) / C::KC;
-  // keys are split until two CTAs sit on every SM, as long as a warp keeps two chunks to itself; 8 is the portable limit
-  int ranks = 1;
-  while (ranks < 8 && items * ranks < 2 * sm_count() && chunks >= 4 * ranks * DC_WARPS) ranks *= 2;
+  int ranks, steps;
+  decode_split(p, D, ranks, steps);
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3(ranks, tiles * p.Hkv, p.B);
   lc.blockDim = dim3(DC_WARPS * 32);

@@ -382,6 +382,24 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 using namespace gb;
 
+// A few query rows: the decoding kernel reads K and V once per 16 rows of a group and splits the keys between CTAs; the tiled
+// kernel has the faster tensor cores and reads them once per head, 128 rows or not.  Which is faster depends on how both fill
+// the GPU, so both times are estimated (us): a start, and per round of CTAs (two on an SM for the decoding kernel) a fixed
+// part and the keys a CTA walks through.  Fitted to 2124 shapes (1 to 64 rows of a group, 16 to 16384 keys, 2 to 4096 KV heads
+// x batch, inputs cycled past L2), where the choice is 0.3 % off the better of the two on average.  Decoding / tiled kernel:
+// 8 x 1 queries, 32 / 4 heads of 128, 4096 keys 19 / 112; 64 x 8, 32 / 4, 1024 keys 82 / 207; one query, 14 / 2 heads of 64, 512
+// keys 8.3 / 10.8; the other way: 256 x 16, 16 / 16 heads of 128, 128 keys 140 / 94; 64 x 16, 4 / 4, 256 keys 22.6 / 16.5.
+static bool decode_wins(const AttnParams& p, int D) {
+  const long long sms = sm_count(), rows = (long long)p.S * (p.Hq / p.Hkv);
+  int ranks, steps;
+  decode_split(p, D, ranks, steps);
+  const long long waves = ((rows + 15) / 16 * p.Hkv * p.B * ranks + 2 * sms - 1) / (2 * sms);
+  const long long rounds = ((long long)p.B * p.Hq + sms - 1) / sms, tiles = (p.Sk + AT_BN - 1) / AT_BN;
+  const double r = rows < 16 ? (double)rows : 16.0;
+  if (D == 64) return 1.5 + waves * (4.8 + 0.87 * steps + 0.05 * r) < 5.8 + rounds * (1.28 + 1.26 * tiles);
+  return 0.9 + waves * (6.25 + 0.86 * steps + 0.11 * r) < 5.7 + rounds * (1.5 + 1.63 * tiles);
+}
+
 extern "C" int gb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S, int Sk,
                            int Hq, int Hkv, int D, int causal, float scale, int is_bf16, int* status,
                            cudaStream_t st) {
@@ -390,15 +408,7 @@ extern "C" int gb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   AttnParams p{};
   p.o = o; p.lse = lse; p.status = status; p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
   p.causal = causal; p.is_bf16 = is_bf16; p.scale = scale;
-  // A few query rows: the decoding kernel reads K and V once per 16 rows of a group and splits the keys, the tiled kernel
-  // reads them once per head and does not.  Up to 16 rows it always wins (107 -> 19 us for 8 x 1 queries, 32 / 4 heads of
-  // 128, 4096 keys; 8.4 -> 6.8 us for one query and 64 keys).  Up to 64 it does where it reads no more often than the
-  // tiled kernel (64 x 8 queries, 32 / 4 heads, 1024 keys: 83 us against 244) or where the tiled grid leaves half the GPU idle
-  // (8 x 64, 4 / 4 heads, 4096 keys: 29 against 58), and loses elsewhere (64 x 64, 4 / 4 heads, 1024 keys: 55 against 27)
-  // and on short keys (8 queries, 32 / 4 heads, 64 keys: 9.8 against 8.4).
-  const long long rows = (long long)S * (Hq / Hkv), passes = (rows + 15) / 16;
-  if ((rows <= 16 || (rows <= 64 && Sk >= 256 && (passes <= Hq / Hkv || 2ll * B * Hq <= sm_count()))) && B <= 65535 &&
-      4 * Hkv <= 65535)
+  if ((long long)S * (Hq / Hkv) <= 64 && B <= 65535 && 4 * Hkv <= 65535 && decode_wins(p, D))
     return attn_decode(q, k, v, p, D, st);
   CUtensorMap tq, tk, tv, to;
   int r;

@@ -60,9 +60,15 @@ FWD = [
     # B, S, Sk, Hq, Hkv, D: one tile and its neighbours, one row more than a pair, ragged keys, enough work for pairs
     (1, 127, 127, 2, 1, 64), (1, 129, 129, 9, 3, 64), (1, 255, 300, 2, 2, 128), (2, 257, 257, 4, 2, 128),
     (1, 385, 1000, 14, 2, 64), (3, 640, 640, 40, 8, 64), (2, 513, 513, 80, 16, 128), (40, 130, 131, 4, 4, 64),
-    # a few query rows: one, a full 16-row tile, one more, the largest that the decoding kernel takes, and the first past it
-    (1, 1, 1, 1, 1, 64), (2, 1, 17, 8, 1, 128), (3, 2, 1030, 16, 2, 64), (1, 17, 100, 1, 1, 128), (2, 5, 4099, 12, 2, 128),
-    (1, 64, 64, 2, 2, 64), (1, 65, 65, 2, 2, 64), (9, 1, 513, 32, 4, 128), (1, 4, 333, 64, 4, 64),
+    # pairs of q tiles that save a round, and an odd tile among them
+    (48, 200, 200, 2, 2, 64), (13, 300, 300, 8, 4, 128),
+    # up to 64 query rows of a group: estimates choose between the decoding kernel (one query, a full 16-row tile, several
+    # tiles of one head, keys shared by CTAs of a cluster) ...
+    (1, 1, 1, 1, 1, 64), (2, 1, 17, 8, 1, 128), (3, 2, 1030, 16, 2, 64), (2, 5, 4099, 12, 2, 128), (9, 1, 513, 32, 4, 128),
+    (1, 4, 333, 64, 4, 64), (1, 17, 300, 1, 1, 128), (1, 64, 300, 2, 2, 64), (2, 64, 1000, 4, 4, 128), (1, 33, 2050, 1, 1, 64),
+    # ... and the tiled one (few keys, many heads), which takes everything from 65 rows on
+    (1, 17, 100, 1, 1, 128), (1, 64, 64, 2, 2, 64), (2, 16, 128, 4, 4, 128), (64, 16, 200, 4, 4, 128), (1, 65, 65, 2, 2, 64),
+    (1, 65, 300, 2, 2, 64), (2, 22, 300, 6, 2, 128),
 ]
 
 
