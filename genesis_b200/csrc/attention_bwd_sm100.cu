@@ -1,9 +1,9 @@
 // Flash-attention backward for sm_100a (tcgen05 / TMEM / TMA): row statistics, dQ kernel, dK/dV kernel.
 //
-// Both kernels work on 128 x 128 score tiles with eight arithmetic warps: two warpgroups share a tile by columns (64
-// each), every thread owns one row of its half (one TMEM lane).  A TMA warp feeds a ring of operand tiles, an MMA warp
-// issues.  P and dS never pass through shared memory: they are written as 16-bit pairs into tensor memory, as the A
-// operand of the GEMM that consumes them.
+// Both kernels work on score tiles of 128 rows and 128 columns (64 where half_tiles says so) with eight arithmetic warps: two
+// warpgroups share a tile by columns, every thread owns one row of its half (one TMEM lane).  A TMA warp feeds a ring of
+// operand tiles, an MMA warp issues.  P and dS never pass through shared memory: they are written as 16-bit pairs into tensor
+// memory, as the A operand of the GEMM that consumes them.
 //   dQ    : CTA = (q tile of 128 rows, head); loop over kv tiles:
 //           S = Q K^T, dP = dO V^T, dS = P o (dP - delta) * scale, dQ += dS K          (K tile reused MN-major)
 //           S and dP of tile j + 1 are issued as soon as those of tile j are in registers, ahead of dQ(j).
@@ -14,9 +14,10 @@
 //           while they exponentiate S^T(i + 1) the tensor cores run dK(i) and dP^T(i + 1).
 // What bounds them: 3 + 4 GEMMs of 128 x 128 x D per score tile (each 512 clocks at D = 128, 256 at D = 64, at the nominal
 // rate) against one exponential per score in each kernel (1024 clocks): the tensor pipe at D = 128, the exponentials at D = 64.
-// Measured against the kernels they replace (128 x 64 tiles, four arithmetic warps, one dK/dV CTA per query head with fp32
-// atomics for every group), whole backward pass, bf16 causal, us: 8 x 2048, 14 / 2 heads of 64: 538 -> 324; 4 x 4096,
-// 12 / 2 of 128: 1437 -> 680; 8 x 1024, 16 / 4 of 128: 436 -> 180; 1 x 1003, 14 / 2 of 64: 80 -> 56.
+// Measured against the kernels they replace (128 x 64 tiles, four arithmetic warps, at D = 64 two CTAs on an SM, one dK/dV CTA
+// per query head with fp32 atomics for every group), whole backward pass, bf16 causal, us: 8 x 2048, 14 / 2 heads of 64:
+// 543 -> 287; 4 x 4096, 12 / 2 of 128: 1444 -> 680; 8 x 1024, 16 / 4 of 128: 430 -> 178; 1 x 1003, 14 / 2 of 64: 69 -> 48;
+// 64 x 197, 12 / 12 of 64: 125 -> 115; 512 x 64, 8 / 8 of 64: 168 -> 173.
 // Reference counterpart: genesis/nn/attention.py:162-406 (Triton, 32 x 32 tiles, Hq == Hkv only).
 #include "attention_common.cuh"
 
@@ -24,13 +25,28 @@ namespace gb {
 
 constexpr int BW_THREADS = 320;     // 2 x 4 arithmetic warps, TMA warp, MMA warp
 
-template <int D> struct BwdCfg {
+// CN: columns of a score tile.  128, or 64 for short rows (see half_tiles): at D = 64 the half tiles leave room for two CTAs on
+// an SM, in tensor memory (256 columns each) and in shared memory.
+template <int D, int CN> struct BwdCfg {
   static constexpr int TILE = AT_BM * D * 2;                    // one [128 x D] 16-bit tile
-  static constexpr int ST = D == 64 ? 3 : 2;                    // stages of the operand ring (two tiles each)
-  static constexpr int STATS = 2 * AT_BM * 4;                   // -lse (log2 domain) and -delta of a q tile
-  static constexpr int SMEM_DQ = 2 * TILE + ST * 2 * TILE + 256;
-  static constexpr int SMEM_KV = 2 * TILE + ST * (2 * TILE + STATS) + 256;
+  static constexpr int CTILE = CN * D * 2;                      // one [CN x D] tile: what a score tile's columns come from
+  static constexpr int ST = D == 64 ? 3 : 2;                    // stages of the operand ring (two CN-row tiles each)
+  static constexpr int STATS = 2 * CN * 4;                      // -lse (log2 domain) and -delta of a q tile
+  static constexpr int SMEM_DQ = 2 * TILE + ST * 2 * CTILE + 256;
+  static constexpr int SMEM_KV = 2 * TILE + ST * (2 * CTILE + STATS) + 256;
+  static constexpr int TM_DQ = CN * 5 / 2 + D <= 256 ? 256 : 512;   // tensor-memory columns: S, dP, dS (16-bit), dQ
+  static constexpr int TM_KV = 2 * CN + 2 * D <= 256 ? 256 : 512;   // S^T, dP^T, dV, dK
+  static constexpr int CTAS = D == 64 && CN == 64 ? 2 : 1;          // on an SM
 };
+
+// HC consecutive fp32 columns of a lane (32 or 64), and HC / 2 packed ones back
+template <int HC> __device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&r)[HC / 32][32]) {
+  tmem_ld_32x32b_x32(addr, r[0]);
+  if constexpr (HC == 64) tmem_ld_32x32b_x32(addr + 32, r[1]);
+  tmem_ld_wait();
+}
+__device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[32]) { tmem_st_32x32b_x32(addr, r); }
+__device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[16]) { tmem_st_32x32b_x16(addr, r); }
 
 __device__ __forceinline__ void store_out_row(uint16_t* dst, uint32_t tsrc, int ncols, bool valid, int dt,
                                               float mul = 1.f) {
@@ -56,13 +72,13 @@ __device__ __forceinline__ void store_out_row(uint16_t* dst, uint32_t tsrc, int 
 // =====================================================================================================
 // dQ
 // =====================================================================================================
-template <int D, bool BF16>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int D, int CN, bool BF16>
+__global__ void __launch_bounds__(BW_THREADS, BwdCfg<D, CN>::CTAS)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                    const __grid_constant__ CUtensorMap tmv, const __grid_constant__ CUtensorMap tmdo,
                    const AttnParams p) {
-  using C = BwdCfg<D>;
-  constexpr int TILE = C::TILE, ST = C::ST;
+  using C = BwdCfg<D, CN>;
+  constexpr int TILE = C::TILE, CTILE = C::CTILE, ST = C::ST, HC = CN / 2;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (status_poisoned(p.status)) return;
   if ((reinterpret_cast<uintptr_t>(smem_raw) & 1023) != 0) {
@@ -72,7 +88,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
   uint8_t* sQ = smem_raw;
   uint8_t* sdO = sQ + TILE;
   uint8_t* sKV = sdO + TILE;         // ST stages of (K, V)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + ST * 2 * TILE);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + ST * 2 * CTILE);
   uint64_t* qdo_full = bars;
   uint64_t* s_full = bars + 1;
   uint64_t* dp_full = bars + 2;
@@ -92,9 +108,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
   const int kvh = h / (p.Hq / p.Hkv);
   const int m0 = qt * AT_BM;
   const int off = p.Sk - p.S;
-  int n_kv = (p.Sk + AT_BN - 1) / AT_BN;
+  int n_kv = (p.Sk + CN - 1) / CN;
   if (p.causal) {
-    const int lim = (m0 + AT_BM + off + AT_BN - 1) / AT_BN;
+    const int lim = (m0 + AT_BM + off + CN - 1) / CN;
     n_kv = lim < n_kv ? lim : n_kv;
   }
   if (n_kv < 1) n_kv = 1;
@@ -106,12 +122,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, C::TM_DQ); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + 128, tdS = tmem + 256, tdQ = tmem + 320;   // 128 + 128 + 64 + D columns
+  const uint32_t tS = tmem, tdP = tmem + CN, tdS = tmem + 2 * CN, tdQ = tmem + 2 * CN + HC;   // CN + CN + CN / 2 + D columns
 
   if (warp == 8) {
     if (lane == 0) {   // ---------------- TMA ----------------
@@ -122,26 +138,25 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
       for (; j < n_kv; ++j) {
         const int st = j % ST;
         if (!AT_WAIT(&kv_empty[st], ((j / ST) & 1) ^ 1, 40)) break;
-        mbar_expect_tx(&kv_full[st], 2 * TILE);
-        load_tile<D>(sKV + st * 2 * TILE, &tmk, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
-        load_tile<D>(sKV + st * 2 * TILE + TILE, &tmv, &kv_full[st], kvh, j * AT_BN, b, AT_BN);
+        mbar_expect_tx(&kv_full[st], 2 * CTILE);
+        load_tile<D>(sKV + st * 2 * CTILE, &tmk, &kv_full[st], kvh, j * CN, b, CN);
+        load_tile<D>(sKV + st * 2 * CTILE + CTILE, &tmv, &kv_full[st], kvh, j * CN, b, CN);
       }
       if (*abort_flag) { drain_copies(qdo_full, 1, 1); drain_copies(kv_full, ST, j); }
     }
   } else if (warp == 9) {
     // ---------------- MMA: the warp stays converged, one elected lane issues ----------------
     constexpr uint32_t fmt = BF16 ? 1u : 0u;
-    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, AT_BN);
+    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, CN);
     constexpr uint32_t idesc_dq = make_idesc(fmt, 0, 1, AT_BM, D);
     const uint32_t aQ = smem_u32(sQ), adO = smem_u32(sdO), aKV = smem_u32(sKV);
     auto score = [&](uint32_t d, uint32_t a, uint32_t bb, uint64_t* done) {
-      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, AT_BN);
+      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, CN);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t o = (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2;
-          umma_f16(d, da + o, db + o, idesc_s, kk > 0);
-        }
+        for (int kk = 0; kk < D / 16; ++kk)        // (descriptors count 16-byte units)
+          umma_f16(d, da + (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2, db + (kk >> 2) * (CN * 128 / 16) + (kk & 3) * 2,
+                   idesc_s, kk > 0);
         umma_commit(done);
       }
       __syncwarp();
@@ -150,24 +165,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
     if (ok) {
       tc_fence_after_sync();
       score(tS, aQ, aKV, s_full);
-      score(tdP, adO, aKV + TILE, dp_full);
+      score(tdP, adO, aKV + CTILE, dp_full);
     }
     for (int j = 0; ok && j < n_kv; ++j) {
       if (j + 1 < n_kv) {
         const int st = (j + 1) % ST;
         if (!(ok = AT_WAIT_ALL(&kv_full[st], ((j + 1) / ST) & 1, 43) && AT_WAIT_ALL(s_free, j & 1, 44))) break;
         tc_fence_after_sync();
-        score(tS, aQ, aKV + st * 2 * TILE, s_full);
+        score(tS, aQ, aKV + st * 2 * CTILE, s_full);
         if (!(ok = AT_WAIT_ALL(dp_free, j & 1, 45))) break;
         tc_fence_after_sync();
-        score(tdP, adO, aKV + st * 2 * TILE + TILE, dp_full);
+        score(tdP, adO, aKV + st * 2 * CTILE + CTILE, dp_full);
       }
       if (!(ok = AT_WAIT_ALL(ds_ready, j & 1, 46))) break;
       tc_fence_after_sync();
-      const uint64_t dk = desc_mnmajor(aKV + (j % ST) * 2 * TILE, 0, AT_BN);
+      const uint64_t dk = desc_mnmajor(aKV + (j % ST) * 2 * CTILE, 0, CN);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < AT_BN / 16; ++kk)
+        for (int kk = 0; kk < CN / 16; ++kk)
           umma_f16_ts(tdQ, tdS + kk * 8, dk + kk * (2048 / 16), idesc_dq, j > 0 || kk > 0);
         umma_commit(acc_done);
         umma_commit(&kv_empty[j % ST]);
@@ -175,7 +190,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
       __syncwarp();
     }
   } else {
-    const int half = warp >> 2;                          // columns half * 64 .. + 63 of every score tile
+    const int half = warp >> 2;                          // columns half * HC .. + HC - 1 of every score tile
     const int row = m0 + (threadIdx.x & 127);
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
     const float sl2 = p.scale * LOG2E;
@@ -187,28 +202,26 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
     for (int j = 0; j < n_kv; ++j) {
       if (!(ok = AT_WAIT_ALL(s_full, j & 1, 50))) break;
       tc_fence_after_sync();
-      float pr[64];
+      float pr[HC];
       {
-        uint32_t s[2][32];
-        tmem_ld_32x32b_x32(tS + lane_base + half * 64, s[0]);
-        tmem_ld_32x32b_x32(tS + lane_base + half * 64 + 32, s[1]);
-        tmem_ld_wait();
+        uint32_t s[HC / 32][32];
+        tmem_ld_cols<HC>(tS + lane_base + half * HC, s);
         tc_fence_before_sync();
         mbar_arrive(s_free);
-        const int col0 = j * AT_BN;
-        if ((col0 + AT_BN > p.Sk) || (p.causal && (col0 + AT_BN - 1 > m0 + off)) || (m0 + AT_BM > p.S)) {
+        const int col0 = j * CN;
+        if ((col0 + CN > p.Sk) || (p.causal && (col0 + CN - 1 > m0 + off)) || (m0 + AT_BM > p.S)) {
           // masked scores become -inf (probability 0) in a pass of their own: the main loop stays branch-free
           int lim = p.causal ? row + off : p.Sk - 1;            // last visible column of this row
           lim = lim < p.Sk - 1 ? lim : p.Sk - 1;
           if (row >= p.S) lim = -1;
-          lim -= col0 + half * 64;
+          lim -= col0 + half * HC;
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i) s[c][i] = (c * 32 + i <= lim) ? s[c][i] : 0xff800000u;
         }
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) {
+        for (int i = 0; i < HC; i += 2) {
           const float2 x = fma2(make_float2(__uint_as_float(s[i >> 5][i & 31]), __uint_as_float(s[i >> 5][(i & 31) + 1])),
                                 sl2v, nlv);
           pr[i] = fast_exp2(x.x);
@@ -217,15 +230,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
       }
       if (!(ok = AT_WAIT_ALL(dp_full, j & 1, 51))) break;
       tc_fence_after_sync();
-      uint32_t dp[2][32], ds[32];
-      tmem_ld_32x32b_x32(tdP + lane_base + half * 64, dp[0]);
-      tmem_ld_32x32b_x32(tdP + lane_base + half * 64 + 32, dp[1]);
-      tmem_ld_wait();
+      uint32_t dp[HC / 32][32], ds[HC / 2];
+      tmem_ld_cols<HC>(tdP + lane_base + half * HC, dp);
       tc_fence_before_sync();
       mbar_arrive(dp_free);
       // dS = P o (dP - delta) as 16-bit pairs (the softmax scale is applied once, to dQ at the end)
 #pragma unroll
-      for (int i = 0; i < 64; i += 2) {
+      for (int i = 0; i < HC; i += 2) {
         const float2 d = mul2(make_float2(pr[i], pr[i + 1]),
                               add2(make_float2(__uint_as_float(dp[i >> 5][i & 31]), __uint_as_float(dp[i >> 5][(i & 31) + 1])), ndv));
         ds[i / 2] = pack2c<BF16>(d.x, d.y);
@@ -233,7 +244,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
       // dS is single-buffered: the previous tile's dQ MMA has to be done reading it
       if (j > 0 && !(ok = AT_WAIT_ALL(acc_done, (j - 1) & 1, 52))) break;
       tc_fence_after_sync();
-      tmem_st_32x32b_x32(tdS + lane_base + half * 32, ds);
+      tmem_st_cols(tdS + lane_base + half * (HC / 2), ds);
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(ds_ready);
@@ -246,7 +257,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
+  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, C::TM_DQ); }
 }
 
 // =====================================================================================================
@@ -254,13 +265,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constan
 // splits == 1 the CTA owns its output rows and stores them; otherwise (too few kv tiles to fill the GPU with whole
 // groups) the parts are added into an fp32 workspace with vector atomics.
 // =====================================================================================================
-template <int D, bool BF16>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int D, int CN, bool BF16>
+__global__ void __launch_bounds__(BW_THREADS, BwdCfg<D, CN>::CTAS)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
                      const __grid_constant__ CUtensorMap tmv, const __grid_constant__ CUtensorMap tmdo,
                      const AttnParams p, float* __restrict__ ws, const int splits) {
-  using C = BwdCfg<D>;
-  constexpr int TILE = C::TILE, ST = C::ST, STAGE = 2 * TILE;
+  using C = BwdCfg<D, CN>;
+  constexpr int TILE = C::TILE, CTILE = C::CTILE, ST = C::ST, STAGE = 2 * CTILE, HC = CN / 2;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (status_poisoned(p.status)) return;
   if ((reinterpret_cast<uintptr_t>(smem_raw) & 1023) != 0) {
@@ -270,7 +281,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
   uint8_t* sK = smem_raw;
   uint8_t* sV = sK + TILE;
   uint8_t* sQ = sV + TILE;           // ST stages of (Q, dO)
-  uint8_t* sStat = sQ + ST * STAGE;  // ST stages of 128 x (-lse), 128 x (-delta)
+  uint8_t* sStat = sQ + ST * STAGE;  // ST stages of CN x (-lse), CN x (-delta)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + ST * C::STATS);
   uint64_t* kv_full = bars;
   uint64_t* s_full = bars + 1;
@@ -290,9 +301,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
   const int kvh = hs / splits, part = hs % splits;
   const int h0 = kvh * group + part * group / splits, h1 = kvh * group + (part + 1) * group / splits;
   const int off = p.Sk - p.S;
-  const int nq = (p.S + AT_BM - 1) / AT_BM;
+  const int nq = (p.S + CN - 1) / CN;
   int i_start = 0;
-  if (p.causal) { const int first = n0 - off; i_start = first > 0 ? first / AT_BM : 0; }
+  if (p.causal) { const int first = n0 - off; i_start = first > 0 ? first / CN : 0; }
   const int nqv = nq > i_start ? nq - i_start : 0;
   const int n_it = nqv * (h1 - h0);
 
@@ -303,12 +314,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, C::TM_KV); tmem_relinquish(); }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 256 + D;
+  const uint32_t tS = tmem, tdP = tmem + CN, tdV = tmem + 2 * CN, tdK = tmem + 2 * CN + D;
 
   if (warp == 8) {
     if (lane == 0 && n_it > 0) {   // ---------------- TMA ----------------
@@ -321,11 +332,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
         const int st = it % ST;
         if (!AT_WAIT(&q_empty[st], ((it / ST) & 1) ^ 1, 60)) break;
         mbar_expect_tx(&q_full[st], STAGE + C::STATS);
-        load_tile<D>(sQ + st * STAGE, &tmq, &q_full[st], h, qt * AT_BM, b, AT_BM);
-        load_tile<D>(sQ + st * STAGE + TILE, &tmdo, &q_full[st], h, qt * AT_BM, b, AT_BM);
-        const float* src = p.stats + ((size_t)b * p.Hq + h) * p.Spad + (size_t)qt * AT_BM;
-        bulk_load(sStat + st * C::STATS, src, AT_BM * 4, &q_full[st]);
-        bulk_load(sStat + st * C::STATS + AT_BM * 4, src + half, AT_BM * 4, &q_full[st]);
+        load_tile<D>(sQ + st * STAGE, &tmq, &q_full[st], h, qt * CN, b, CN);
+        load_tile<D>(sQ + st * STAGE + CTILE, &tmdo, &q_full[st], h, qt * CN, b, CN);
+        const float* src = p.stats + ((size_t)b * p.Hq + h) * p.Spad + (size_t)qt * CN;
+        bulk_load(sStat + st * C::STATS, src, CN * 4, &q_full[st]);
+        bulk_load(sStat + st * C::STATS + CN * 4, src + half, CN * 4, &q_full[st]);
         if (++qt == nq) { qt = i_start; ++h; }
       }
       if (*abort_flag) { drain_copies(kv_full, 1, 1); drain_copies(q_full, ST, it); }
@@ -333,29 +344,28 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
   } else if (warp == 9) {
     // ---------------- MMA: the warp stays converged, one elected lane issues ----------------
     constexpr uint32_t fmt = BF16 ? 1u : 0u;
-    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, AT_BN);
+    constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, AT_BM, CN);
     constexpr uint32_t idesc_acc = make_idesc(fmt, 0, 1, AT_BM, D);
     const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ);
     auto score = [&](uint32_t d, uint32_t a, uint32_t bb, uint64_t* done) {
-      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, AT_BN);
+      const uint64_t da = desc_kmajor(a, 0, AT_BM), db = desc_kmajor(bb, 0, CN);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t o = (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2;
-          umma_f16(d, da + o, db + o, idesc_s, kk > 0);
-        }
+        for (int kk = 0; kk < D / 16; ++kk)        // (descriptors count 16-byte units)
+          umma_f16(d, da + (kk >> 2) * (AT_BM * 128 / 16) + (kk & 3) * 2, db + (kk >> 2) * (CN * 128 / 16) + (kk & 3) * 2,
+                   idesc_s, kk > 0);
         umma_commit(done);
       }
       __syncwarp();
     };
-    // acc (+)= A B: A = 16-bit pairs in tensor memory, columns 0..31 for k < 64 and 64..95 behind them (each
-    // warpgroup packs into the columns it read), B = an operand tile as MN-major
+    // acc (+)= A B: A = 16-bit pairs in tensor memory, the first half of the columns of each half tile (each warpgroup
+    // packs into the columns it read), B = an operand tile as MN-major
     auto accumulate = [&](uint32_t d, uint32_t a, uint32_t tile, bool first) {
-      const uint64_t db = desc_mnmajor(tile, 0, AT_BN);
+      const uint64_t db = desc_mnmajor(tile, 0, CN);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < AT_BN / 16; ++kk)
-          umma_f16_ts(d, a + (kk >> 2) * 64 + (kk & 3) * 8, db + kk * (2048 / 16), idesc_acc, !first || kk > 0);
+        for (int kk = 0; kk < CN / 16; ++kk)
+          umma_f16_ts(d, a + kk / (HC / 16) * HC + kk % (HC / 16) * 8, db + kk * (2048 / 16), idesc_acc, !first || kk > 0);
       }
       __syncwarp();
     };
@@ -363,14 +373,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
     if (ok) {
       tc_fence_after_sync();
       score(tS, aK, aQ, s_full);
-      score(tdP, aV, aQ + TILE, dp_full);
+      score(tdP, aV, aQ + CTILE, dp_full);
     }
     for (int it = 0; ok && it < n_it; ++it) {
       const uint32_t cur = aQ + (it % ST) * STAGE, nxt = aQ + ((it + 1) % ST) * STAGE;
       const bool more = it + 1 < n_it;
       if (!(ok = AT_WAIT_ALL(p_ready, it & 1, 63))) break;
       tc_fence_after_sync();
-      accumulate(tdV, tS, cur + TILE, it == 0);
+      accumulate(tdV, tS, cur + CTILE, it == 0);
       if (more) {
         if (!(ok = AT_WAIT_ALL(&q_full[(it + 1) % ST], ((it + 1) / ST) & 1, 64))) break;
         tc_fence_after_sync();
@@ -381,44 +391,42 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
       accumulate(tdK, tdP, cur, it == 0);
       if (elect_one()) umma_commit(more ? &q_empty[it % ST] : acc_done);
       __syncwarp();
-      if (more) score(tdP, aV, nxt + TILE, dp_full);
+      if (more) score(tdP, aV, nxt + CTILE, dp_full);
     }
   } else {
-    const int half = warp >> 2;                          // columns half * 64 .. + 63 of every score tile
+    const int half = warp >> 2;                          // columns half * HC .. + HC - 1 of every score tile
     const int kvrow = n0 + (threadIdx.x & 127);
     const uint32_t lane_base = ((uint32_t)((warp & 3) * 32)) << 16;
-    const uint32_t tSh = tS + lane_base + half * 64, tdPh = tdP + lane_base + half * 64;
+    const uint32_t tSh = tS + lane_base + half * HC, tdPh = tdP + lane_base + half * HC;
     const float sl2 = p.scale * LOG2E;
     const float2 sl2v = make_float2(sl2, sl2);
     bool ok = true;
     int qt = i_start;
     for (int it = 0; it < n_it; ++it) {
-      const int q0 = qt * AT_BM + half * 64;
+      const int q0 = qt * CN + half * HC;
       if (++qt == nq) qt = i_start;
       const int st = it % ST;
-      const float4* nl = reinterpret_cast<const float4*>(sStat + st * C::STATS + half * 256);
-      const float4* nd = reinterpret_cast<const float4*>(sStat + st * C::STATS + AT_BM * 4 + half * 256);
+      const float4* nl = reinterpret_cast<const float4*>(sStat + st * C::STATS + half * HC * 4);
+      const float4* nd = reinterpret_cast<const float4*>(sStat + st * C::STATS + CN * 4 + half * HC * 4);
       // (the statistics are this stage's own: seen through the barrier that their copy completed on)
       if (!(ok = AT_WAIT_ALL(&q_full[st], (it / ST) & 1, 70) && AT_WAIT_ALL(s_full, it & 1, 71))) break;
       tc_fence_after_sync();
-      float pr[64];
+      float pr[HC];
       {
-        uint32_t s[2][32], pk[32];
-        tmem_ld_32x32b_x32(tSh, s[0]);
-        tmem_ld_32x32b_x32(tSh + 32, s[1]);
-        tmem_ld_wait();
-        if ((q0 + 64 > p.S) || (n0 + AT_BM > p.Sk) || (p.causal && (n0 + AT_BM - 1 > q0 + off))) {
+        uint32_t s[HC / 32][32], pk[HC / 2];
+        tmem_ld_cols<HC>(tSh, s);
+        if ((q0 + HC > p.S) || (n0 + AT_BM > p.Sk) || (p.causal && (n0 + AT_BM - 1 > q0 + off))) {
           // this kv row is visible to query columns first..last of the half tile
           const int first = p.causal ? kvrow - off - q0 : 0;
           const int last = kvrow < p.Sk ? p.S - 1 - q0 : -1;
 #pragma unroll
-          for (int c = 0; c < 2; ++c)
+          for (int c = 0; c < HC / 32; ++c)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               s[c][i] = (c * 32 + i >= first && c * 32 + i <= last) ? s[c][i] : 0xff800000u;   // -inf: probability 0
         }
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
+        for (int i = 0; i < HC; i += 4) {
           const float4 n4 = nl[i / 4];
           const uint32_t* v = &s[i >> 5][i & 31];
           const float2 x = fma2(make_float2(__uint_as_float(v[0]), __uint_as_float(v[1])), sl2v, make_float2(n4.x, n4.y));
@@ -427,19 +435,17 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
           pk[i / 2] = pack2c<BF16>(pr[i], pr[i + 1]);
           pk[i / 2 + 1] = pack2c<BF16>(pr[i + 2], pr[i + 3]);
         }
-        tmem_st_32x32b_x32(tSh, pk);
+        tmem_st_cols(tSh, pk);
       }
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(p_ready);
       if (!(ok = AT_WAIT_ALL(dp_full, it & 1, 72))) break;
       tc_fence_after_sync();
-      uint32_t dp[2][32], ds[32];
-      tmem_ld_32x32b_x32(tdPh, dp[0]);
-      tmem_ld_32x32b_x32(tdPh + 32, dp[1]);
-      tmem_ld_wait();
+      uint32_t dp[HC / 32][32], ds[HC / 2];
+      tmem_ld_cols<HC>(tdPh, dp);
 #pragma unroll
-      for (int i = 0; i < 64; i += 4) {       // (the softmax scale is applied once, to dK at the end)
+      for (int i = 0; i < HC; i += 4) {       // (the softmax scale is applied once, to dK at the end)
         const float4 n4 = nd[i / 4];
         const uint32_t* v = &dp[i >> 5][i & 31];
         const float2 x = mul2(make_float2(pr[i], pr[i + 1]),
@@ -449,7 +455,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
         ds[i / 2] = pack2c<BF16>(x.x, x.y);
         ds[i / 2 + 1] = pack2c<BF16>(y.x, y.y);
       }
-      tmem_st_32x32b_x32(tdPh, ds);
+      tmem_st_cols(tdPh, ds);
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(ds_ready);
@@ -489,7 +495,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, 512); }
+  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem, C::TM_KV); }
 }
 
 // Row statistics of the backward kernels, rows padded to whole q tiles: stats[0][b, h, s] = -lse in the log2 domain (-inf
@@ -557,25 +563,65 @@ static int dkdv_splits(int B, int S, int Sk, int Hq, int Hkv, int causal) {
   return group;
 }
 
+template <int D, int CN, bool BF16>
+static int launch_dkdv(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& dout,
+                       const AttnParams& p, float* ws, int splits, int grid, cudaStream_t st) {
+  static unsigned long long cfg = 0;
+  if (int e = smem_opt_in(attn_bwd_dkdv_kernel<D, CN, BF16>, BwdCfg<D, CN>::SMEM_KV, cfg)) return e;
+  attn_bwd_dkdv_kernel<D, CN, BF16><<<grid, BW_THREADS, BwdCfg<D, CN>::SMEM_KV, st>>>(q, k, v, dout, p, ws, splits);
+  return (int)cudaGetLastError();
+}
+template <int D, int CN, bool BF16>
+static int launch_dq(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const CUtensorMap& dout,
+                     const AttnParams& p, int grid, cudaStream_t st) {
+  static unsigned long long cfg = 0;
+  if (int e = smem_opt_in(attn_bwd_dq_kernel<D, CN, BF16>, BwdCfg<D, CN>::SMEM_DQ, cfg)) return e;
+  attn_bwd_dq_kernel<D, CN, BF16><<<grid, BW_THREADS, BwdCfg<D, CN>::SMEM_DQ, st>>>(q, k, v, dout, p);
+  return (int)cudaGetLastError();
+}
+
+// Whether a kernel of `grid` CTAs, the longest of which walks through `length` whole score tiles whose columns come from
+// sequences of `cols` rows, takes half tiles.  Where the columns fit one, the other half would be padding: 128 x 16, 12 / 12
+// heads of 128 135 -> 113 us, 32 x 64, 16 / 16 61 -> 52.  At D = 64 half tiles put two CTAs on an SM, and one's start, epilogue
+// and waits are under the other's arithmetic: they win as soon as there are enough CTAs.  Backward pass with whole tiles /
+// half tiles, causal, us: 16 / 16 heads, 128 x 64 164 / 92, 128 x 128 193 / 130, 32 x 512 236 / 170, 8 x 1024 150 / 118; 14 / 2
+// heads, 8 x 2048 326 / 287.  A CTA that has its SM to itself is faster on whole ones (1 x 1536, 16 / 16 45 / 55), and with less
+// than two CTAs for every SM the longest one decides, so there only short ones split.  (1750 shapes: 0.8 % off the better
+// of the two on average.)
+static bool half_tiles(long long grid, int cols, int length, int D) {
+  if (cols <= 64) return true;
+  return D == 64 && (grid > 2 * sm_count() || (grid > sm_count() && length <= 8));
+}
+
 template <typename T, int D, bool BF16>
-static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                      const AttnParams& p, const void* o, const void* dout, const float* lse, float* stats, float* ws,
-                      int splits, cudaStream_t st) {
-  using C = BwdCfg<D>;
-  static unsigned long long cfg_dq = 0, cfg_kv = 0;
-  int r;
-  if ((r = smem_opt_in(attn_bwd_dq_kernel<D, BF16>, C::SMEM_DQ, cfg_dq)) != 0) return r;
-  if ((r = smem_opt_in(attn_bwd_dkdv_kernel<D, BF16>, C::SMEM_KV, cfg_kv)) != 0) return r;
+static int launch_bwd(const AttnParams& p, const void* q, const void* k, const void* v, const void* o, const void* dout,
+                      const float* lse, float* stats, float* ws, int splits, cudaStream_t st) {
   const long long gq = (long long)((p.S + AT_BM - 1) / AT_BM) * p.Hq * p.B;
   const long long gk = (long long)((p.Sk + AT_BM - 1) / AT_BM) * p.Hkv * splits * p.B;
   if (gq > 0x7fffffff || gk > 0x7fffffff) return -5;
+  // tiles of 128 rows, and of 64 where they are the columns of half score tiles
+  CUtensorMap tq, tk, tv, tdo, hq, hk, hv, hdo;
+  const int group = p.Hq / p.Hkv;
+  const bool nq = half_tiles(gq, p.Sk, (p.Sk + AT_BN - 1) / AT_BN, D);
+  const bool nk = half_tiles(gk, p.S, (p.S + AT_BN - 1) / AT_BN * ((group + splits - 1) / splits), D);
+  auto map = [&](CUtensorMap& m, const void* t, int S, int H, int rows) {
+    return make_tmap_bshd(&m, t, BF16 ? 1 : 0, p.B, S, H, D, rows);
+  };
+  int r;
+  if ((r = map(tq, q, p.S, p.Hq, 128)) != 0 || (nk && (r = map(hq, q, p.S, p.Hq, 64)) != 0)) return 10000 + r;
+  if ((r = map(tk, k, p.Sk, p.Hkv, 128)) != 0 || (nq && (r = map(hk, k, p.Sk, p.Hkv, 64)) != 0)) return 20000 + r;
+  if ((r = map(tv, v, p.Sk, p.Hkv, 128)) != 0 || (nq && (r = map(hv, v, p.Sk, p.Hkv, 64)) != 0)) return 30000 + r;
+  if ((r = map(tdo, dout, p.S, p.Hq, 128)) != 0 || (nk && (r = map(hdo, dout, p.S, p.Hq, 64)) != 0)) return 40000 + r;
   const long long lanes = (long long)p.B * p.Spad * p.Hq * (D / 8), nkv = (long long)p.B * p.Sk * p.Hkv * D;
   attn_stats_kernel<T, D><<<gb_grid(lanes, 256), 256, 0, st>>>((const T*)o, (const T*)dout, lse, stats, p.B, p.S,
                                                                p.Spad, p.Hq);
   if (splits > 1 && (r = (int)cudaMemsetAsync(ws, 0, 2 * nkv * sizeof(float), st)) != 0) return r;
-  attn_bwd_dkdv_kernel<D, BF16><<<(int)gk, BW_THREADS, C::SMEM_KV, st>>>(tq, tk, tv, tdo, p, splits > 1 ? ws : nullptr,
-                                                                        splits);
-  attn_bwd_dq_kernel<D, BF16><<<(int)gq, BW_THREADS, C::SMEM_DQ, st>>>(tq, tk, tv, tdo, p);
+  if (splits == 1) ws = nullptr;
+  r = nk ? launch_dkdv<D, 64, BF16>(hq, tk, tv, hdo, p, ws, splits, (int)gk, st)
+         : launch_dkdv<D, 128, BF16>(tq, tk, tv, tdo, p, ws, splits, (int)gk, st);
+  if (r != 0) return r;
+  r = nq ? launch_dq<D, 64, BF16>(tq, hk, hv, tdo, p, (int)gq, st) : launch_dq<D, 128, BF16>(tq, tk, tv, tdo, p, (int)gq, st);
+  if (r != 0) return r;
   if (splits > 1)
     attn_dkv_convert_kernel<T><<<gb_grid(nkv / 2, 256), 256, 0, st>>>(ws, (T*)p.dk, (T*)p.dv, nkv);
   return (int)cudaGetLastError();
@@ -599,12 +645,6 @@ extern "C" int gb_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (D != 64 && D != 128) return -2;
   if (Hq % Hkv != 0 || Sk < S) return -3;
   if (scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) != 0) return -4;
-  CUtensorMap tq, tk, tv, tdo;
-  int r;
-  if ((r = make_tmap_bshd(&tq, q, is_bf16, B, S, Hq, D)) != 0) return 10000 + r;
-  if ((r = make_tmap_bshd(&tk, k, is_bf16, B, Sk, Hkv, D)) != 0) return 20000 + r;
-  if ((r = make_tmap_bshd(&tv, v, is_bf16, B, Sk, Hkv, D)) != 0) return 30000 + r;
-  if ((r = make_tmap_bshd(&tdo, dout, is_bf16, B, S, Hq, D)) != 0) return 40000 + r;
   AttnParams p{};
   p.Spad = (S + AT_BM - 1) / AT_BM * AT_BM;
   p.stats = scratch; p.dq = dq; p.dk = dk; p.dv = dv; p.status = status;
@@ -612,8 +652,8 @@ extern "C" int gb_attn_bwd(const void* q, const void* k, const void* v, const vo
   float* ws = scratch + 2 * (long long)B * Hq * p.Spad;
   const int splits = dkdv_splits(B, S, Sk, Hq, Hkv, causal);
   if (D == 64)
-    return is_bf16 ? launch_bwd<__nv_bfloat16, 64, true>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st)
-                   : launch_bwd<__half, 64, false>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st);
-  return is_bf16 ? launch_bwd<__nv_bfloat16, 128, true>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st)
-                 : launch_bwd<__half, 128, false>(tq, tk, tv, tdo, p, o, dout, lse, scratch, ws, splits, st);
+    return is_bf16 ? launch_bwd<__nv_bfloat16, 64, true>(p, q, k, v, o, dout, lse, scratch, ws, splits, st)
+                   : launch_bwd<__half, 64, false>(p, q, k, v, o, dout, lse, scratch, ws, splits, st);
+  return is_bf16 ? launch_bwd<__nv_bfloat16, 128, true>(p, q, k, v, o, dout, lse, scratch, ws, splits, st)
+                 : launch_bwd<__half, 128, false>(p, q, k, v, o, dout, lse, scratch, ws, splits, st);
 }

@@ -116,6 +116,10 @@ BWD = [
     (1, 127, 127, 2, 1, 64), (1, 129, 130, 4, 2, 128), (2, 256, 256, 6, 3, 64), (1, 385, 500, 14, 2, 64),
     (1, 40, 700, 4, 1, 128), (4, 520, 520, 12, 2, 128), (8, 650, 650, 14, 2, 64), (2, 384, 384, 5, 5, 128),
     (1, 1, 1, 2, 1, 64), (1, 3, 260, 6, 2, 128),
+    # half tiles: rows that fit one and the first that do not, grids on both sides of one and two CTAs for every SM, groups
+    # that are split or not, keys that few queries see
+    (1, 64, 64, 2, 2, 128), (1, 65, 65, 2, 2, 128), (3, 50, 200, 4, 2, 128), (8, 16, 216, 16, 8, 64), (150, 16, 16, 2, 1, 64),
+    (10, 129, 129, 8, 8, 64), (9, 129, 192, 8, 8, 64), (40, 130, 130, 8, 8, 64), (19, 300, 700, 8, 8, 64), (30, 193, 193, 14, 2, 64),
 ]
 
 
