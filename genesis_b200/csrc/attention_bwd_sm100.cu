@@ -16,8 +16,8 @@
 // rate) against one exponential per score in each kernel (1024 clocks): the tensor pipe at D = 128, the exponentials at D = 64.
 // Measured against the kernels they replace (128 x 64 tiles, four arithmetic warps, at D = 64 two CTAs on an SM, one dK/dV CTA
 // per query head with fp32 atomics for every group), whole backward pass, bf16 causal, us: 8 x 2048, 14 / 2 heads of 64:
-// 543 -> 287; 4 x 4096, 12 / 2 of 128: 1444 -> 680; 8 x 1024, 16 / 4 of 128: 430 -> 178; 1 x 1003, 14 / 2 of 64: 69 -> 48;
-// 64 x 197, 12 / 12 of 64: 125 -> 115; 512 x 64, 8 / 8 of 64: 168 -> 173.
+// 543 -> 281; 4 x 4096, 12 / 2 of 128: 1444 -> 676; 8 x 1024, 16 / 4 of 128: 430 -> 174; 1 x 1003, 14 / 2 of 64: 69 -> 48;
+// 64 x 197, 12 / 12 of 64: 125 -> 113; 512 x 64, 8 / 8 of 64: 168 -> 163.
 // Reference counterpart: genesis/nn/attention.py:162-406 (Triton, 32 x 32 tiles, Hq == Hkv only).
 #include "attention_common.cuh"
 
@@ -499,24 +499,23 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_const
 }
 
 // Row statistics of the backward kernels, rows padded to whole q tiles: stats[0][b, h, s] = -lse in the log2 domain (-inf
-// behind the last row: probability 0), stats[1][b, h, s] = -sum_d dO * O.  D / 8 lanes per row, 16 bytes per lane.
+// behind the last row: probability 0), stats[1][b, h, s] = -sum_d dO * O.  D / 8 lanes per row, 16 bytes per lane; the lanes
+// of row s also write the padding of rows S + s, 2 S + s, ...  (With rows of their own for the padding, and 64-bit indices, the
+// backward of 128 x 16 rows, 16 / 16 heads of 64 took 86 us instead of 76.  No GPU holds 2^31 rows of 128 bytes and more.)
 template <typename T, int D>
 __global__ void attn_stats_kernel(const T* __restrict__ o, const T* __restrict__ dout, const float* __restrict__ lse,
-                                  float* __restrict__ stats, int B, int S, int Spad, int H) {
-  constexpr int LPR = D / 8;                 // lanes per row (8 or 16)
-  const long long rows = (long long)B * Spad * H;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  const int sub = (int)(tid % LPR);
+                                  float* __restrict__ stats, unsigned B, unsigned S, unsigned Spad, unsigned H) {
+  constexpr unsigned LPR = D / 8;            // lanes per row (8 or 16)
+  const unsigned rows = B * S * H;
+  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x / LPR;
+  const unsigned sub = tid % LPR;
   // whole warps leave the loop together: rows per pass is a multiple of the rows a warp covers
-  for (long long r0 = tid / LPR; r0 - (threadIdx.x & 31) / LPR < rows; r0 += nthreads / LPR) {
-    const int h = (int)(r0 % H);
-    const long long bs = r0 / H;
-    const int s = (int)(bs % Spad), b = (int)(bs / Spad);
-    const bool live = r0 < rows && s < S;
+  for (unsigned r0 = tid / LPR; r0 - (threadIdx.x & 31) / LPR < rows; r0 += step) {
+    const unsigned h = r0 % H, bs = r0 / H, s = bs % S, b = bs / S;
+    const bool live = r0 < rows;
     float acc = 0.f;
     if (live) {
-      const long long at = (((long long)b * S + s) * H + h) * D + sub * 8;
+      const long long at = (long long)r0 * D + sub * 8;
       const Vec16<T> a = ld16(o + at);
       const Vec16<T> g = ld16(dout + at);
 #pragma unroll
@@ -524,10 +523,16 @@ __global__ void attn_stats_kernel(const T* __restrict__ o, const T* __restrict__
     }
 #pragma unroll
     for (int m = LPR / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if (sub == 0 && r0 < rows) {
-      const long long at = ((long long)b * H + h) * Spad + s;
-      stats[at] = live ? -lse[((long long)b * H + h) * S + s] * LOG2E : -INFINITY;
-      stats[rows + at] = live ? -acc : 0.f;
+    if (live) {
+      const size_t head = (size_t)(b * H + h) * Spad, half = (size_t)B * H * Spad;
+      if (sub == 0) {
+        stats[head + s] = -lse[(size_t)(b * H + h) * S + s] * LOG2E;
+        stats[half + head + s] = -acc;
+      }
+      for (unsigned pad = S + s + sub * S; pad < Spad; pad += LPR * S) {
+        stats[head + pad] = -INFINITY;
+        stats[half + head + pad] = 0.f;
+      }
     }
   }
 }
@@ -612,7 +617,7 @@ static int launch_bwd(const AttnParams& p, const void* q, const void* k, const v
   if ((r = map(tk, k, p.Sk, p.Hkv, 128)) != 0 || (nq && (r = map(hk, k, p.Sk, p.Hkv, 64)) != 0)) return 20000 + r;
   if ((r = map(tv, v, p.Sk, p.Hkv, 128)) != 0 || (nq && (r = map(hv, v, p.Sk, p.Hkv, 64)) != 0)) return 30000 + r;
   if ((r = map(tdo, dout, p.S, p.Hq, 128)) != 0 || (nk && (r = map(hdo, dout, p.S, p.Hq, 64)) != 0)) return 40000 + r;
-  const long long lanes = (long long)p.B * p.Spad * p.Hq * (D / 8), nkv = (long long)p.B * p.Sk * p.Hkv * D;
+  const long long lanes = (long long)p.B * p.S * p.Hq * (D / 8), nkv = (long long)p.B * p.Sk * p.Hkv * D;
   attn_stats_kernel<T, D><<<gb_grid(lanes, 256), 256, 0, st>>>((const T*)o, (const T*)dout, lse, stats, p.B, p.S,
                                                                p.Spad, p.Hq);
   if (splits > 1 && (r = (int)cudaMemsetAsync(ws, 0, 2 * nkv * sizeof(float), st)) != 0) return r;
