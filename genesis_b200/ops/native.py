@@ -879,7 +879,8 @@ def _wdt(x, w):
 
 def rmsnorm_fwd(x, w, eps):
     cols = x.shape[-1]
-    if not _norm_ok(x, cols) or _wdt(x, w) is None or not _weights_ok(x, w, cols):
+    wdt = _wdt(x, w)
+    if wdt is None or not _norm_ok(x, cols) or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     y = torch.empty_like(x)
@@ -887,26 +888,27 @@ def rmsnorm_fwd(x, w, eps):
     if 8192 <= cols * x.element_size() <= 65536 and rows >= 64:
         # wide rows: streamed through shared memory with the next row's copy in flight (csrc/row_stream.cuh)
         rc = lib().gb_rmsnorm_fwd_stream(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rows, cols,
-                                         float(eps), _DT[x.dtype], _wdt(x, w), status_tensor(x.device).data_ptr(), _st())
+                                         float(eps), _DT[x.dtype], wdt, status_tensor(x.device).data_ptr(), _st())
         if rc != -9:
             _chk(rc, "rmsnorm_fwd_stream")
             return y, rstd
     _chk(lib().gb_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rows, cols, float(eps),
-                              _DT[x.dtype], _wdt(x, w), _st()), "rmsnorm_fwd")
+                              _DT[x.dtype], wdt, _st()), "rmsnorm_fwd")
     return y, rstd
 
 
 def add_rmsnorm_fwd(x, res, w, eps):
     """(s = x + res, rmsnorm(s) * w, rstd) in one pass over the rows."""
     cols = x.shape[-1]
+    wdt = _wdt(x, w)
     if not _norm_ok(x, cols) or not _norm_ok(res, cols) or res.dtype != x.dtype or res.shape != x.shape \
-            or _wdt(x, w) is None or not _weights_ok(x, w, cols):
+            or wdt is None or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     s, y = torch.empty_like(x), torch.empty_like(x)
     rstd = torch.empty(rows, dtype=F32, device=x.device)
     _chk(lib().gb_add_rmsnorm_fwd(x.data_ptr(), res.data_ptr(), s.data_ptr(), w.data_ptr(), y.data_ptr(),
-                                  rstd.data_ptr(), rows, cols, float(eps), _DT[x.dtype], _wdt(x, w),
+                                  rstd.data_ptr(), rows, cols, float(eps), _DT[x.dtype], wdt,
                                   status_tensor(x.device).data_ptr(), _st()), "add_rmsnorm_fwd")
     return s, y, rstd
 
@@ -914,8 +916,9 @@ def add_rmsnorm_fwd(x, res, w, eps):
 def add_rmsnorm_bwd(g, gres, x, w, rstd):
     """(rmsnorm_backward(g) + gres, dw): the gradient of either addend of the sum that was normalised."""
     cols = x.shape[-1]
+    wdt = _wdt(x, w)
     if not _norm_ok(x, cols) or not _norm_ok(g, cols) or not _norm_ok(gres, cols) or g.dtype != x.dtype \
-            or gres.dtype != x.dtype or _wdt(x, w) is None or not _weights_ok(x, w, cols):
+            or gres.dtype != x.dtype or wdt is None or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
     L = lib()
@@ -923,7 +926,7 @@ def add_rmsnorm_bwd(g, gres, x, w, rstd):
     dx = torch.empty_like(x)
     part = torch.empty(nct * cols, dtype=F32, device=x.device)
     _chk(L.gb_add_rmsnorm_bwd(g.data_ptr(), gres.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(),
-                              dx.data_ptr(), part.data_ptr(), rows, cols, _DT[x.dtype], _wdt(x, w),
+                              dx.data_ptr(), part.data_ptr(), rows, cols, _DT[x.dtype], wdt,
                               status_tensor(x.device).data_ptr(), _st()), "add_rmsnorm_bwd")
     return dx, _colsum(part, nct, cols)
 
@@ -934,7 +937,8 @@ def _colsum(partial, nrows, cols):
 
 def rmsnorm_bwd(g, x, w, rstd):
     cols = x.shape[-1]
-    if not _norm_ok(x, cols) or not _norm_ok(g, cols) or g.dtype != x.dtype or _wdt(x, w) is None \
+    wdt = _wdt(x, w)
+    if not _norm_ok(x, cols) or not _norm_ok(g, cols) or g.dtype != x.dtype or wdt is None \
             or not _weights_ok(x, w, cols):
         return NotImplemented
     rows = x.numel() // cols
@@ -943,7 +947,7 @@ def rmsnorm_bwd(g, x, w, rstd):
     dx = torch.empty_like(x)
     part = torch.empty(nct * cols, dtype=F32, device=x.device)
     _chk(L.gb_rmsnorm_bwd(g.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), part.data_ptr(),
-                          rows, cols, _DT[x.dtype], _wdt(x, w), status_tensor(x.device).data_ptr(), _st()),
+                          rows, cols, _DT[x.dtype], wdt, status_tensor(x.device).data_ptr(), _st()),
          "rmsnorm_bwd")
     return dx, _colsum(part, nct, cols)
 
