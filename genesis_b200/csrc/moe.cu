@@ -6,6 +6,7 @@
 //   sort           : counting sort of the (token, slot) pairs by expert into segments padded to a
 //                    multiple of `align` rows (what the grouped GEMM consumes); replaces the reference's
 //                    argsort = N sequential launches (tensor_ops.py:236-322)
+#include <type_traits>
 #include "common.cuh"
 
 namespace gb {
@@ -186,23 +187,28 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
 }
 
 // backward of combine: dy[pos[t,j], :] = w[t,j] * g[t, :];  dw[t,j] = <g[t,:], y[pos[t,j],:]>
-// One warp per (token, slot), 16 bytes per lane: y is read and dy written once; the k warps of a token sit in one CTA,
-// so its row of g comes from L1 after the first of them.  4096 tokens x 8 x 2048 bf16: 91 us with two bytes per lane -> 49 us.
-template <typename T>
+// LPR lanes per (token, slot), 16 bytes per lane: y is read and dy written once; the k groups of a token sit in one CTA, so
+// its row of g comes from L1 after the first of them.  With `row_token` (negative where no token was sorted to) the same
+// launch zeroes the rows without a token.  bf16, with the zeroing, two bytes per lane behind a memset -> this: 4096 tokens x 8
+// x 2048 132 -> 59 us.  Rows of less than 32 vectors take groups of 8 or 16 lanes: 65536 x 8 x 64 115 us with two bytes per
+// lane, 148 with a warp of which 8 lanes work, 53 with 8 lanes per row; one token 6.2, 7.2 (two launches), 4.2.
+template <typename T, int LPR>
 __global__ void moe_combine_bwd_vec_kernel(const T* __restrict__ g, const T* __restrict__ y, const float* __restrict__ w,
-                                           const int* __restrict__ pos, T* __restrict__ dy, float* __restrict__ dw,
-                                           long long tokens, int k, int cols) {
+                                           const int* __restrict__ pos, const int* __restrict__ row_token,
+                                           T* __restrict__ dy, float* __restrict__ dw, long long tokens, long long rows,
+                                           int k, int cols) {
   constexpr int V = Vec16<T>::N;
-  const int lane = threadIdx.x & 31, nv = cols / V;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long pr = warp; pr < tokens * k; pr += nwarps) {
+  const int lane = threadIdx.x % LPR, nv = cols / V;
+  const unsigned mask = LPR == 32 ? 0xffffffffu : ((1u << (LPR % 32)) - 1) << (threadIdx.x % 32 / LPR * LPR);
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+  const long long step = (long long)gridDim.x * blockDim.x / LPR;
+  for (long long pr = first; pr < tokens * k; pr += step) {
     const T* gr = g + pr / k * cols;
     const long long row = (long long)pos[pr] * cols;
     const float ws = w[pr];
     float dot = 0.f;
 #pragma unroll 4
-    for (int c = lane; c < nv; c += 32) {
+    for (int c = lane; c < nv; c += LPR) {
       const Vec16<T> a = ld16(gr + c * V), b = ld16(y + row + c * V);
       Vec16<T> o;
 #pragma unroll
@@ -213,20 +219,16 @@ __global__ void moe_combine_bwd_vec_kernel(const T* __restrict__ g, const T* __r
       }
       st16(dy + row + c * V, o);
     }
-    dot = warp_sum(dot);
+#pragma unroll
+    for (int m = LPR / 2; m > 0; m >>= 1) dot += __shfl_xor_sync(mask, dot, m);
     if (lane == 0) dw[pr] = dot;
   }
-}
-
-// zeroes the rows of `dst` that no token was sorted into (row_token < 0); one warp per row
-__global__ void moe_zero_pads_kernel(const int* __restrict__ row_token, uint4* __restrict__ dst, long long rows,
-                                     int vec_per_row) {
-  const int lane = threadIdx.x & 31;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarps) {
-    if (row_token[r] >= 0) continue;
-    for (int c = lane; c < vec_per_row; c += 32) dst[r * vec_per_row + c] = make_uint4(0, 0, 0, 0);
-  }
+  if (row_token != nullptr)
+    for (long long r = first; r < rows; r += step) {
+      if (row_token[r] >= 0) continue;
+      uint4* d = reinterpret_cast<uint4*>(dy + r * cols);
+      for (int c = lane; c < nv; c += LPR) d[c] = make_uint4(0, 0, 0, 0);
+    }
 }
 
 // the same for rows that are not whole 16-byte vectors
@@ -309,16 +311,22 @@ extern "C" int gb_moe_combine_bwd(const void* g, const void* y, const float* w, 
   const int es = dt == DT_F32 ? 4 : 2;
   const bool vec = (long long)cols * es % 16 == 0 &&
                    ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dy)) & 15) == 0;
-  if (row_token != nullptr && rows > 0) {
-    if (!vec) return -2;
-    moe_zero_pads_kernel<<<gb_grid(rows * 32, 256), 256, 0, st>>>(row_token, (uint4*)dy, rows, cols * es / 16);
-  }
-  if (tokens == 0) return (int)cudaGetLastError();
+  if (row_token != nullptr && !vec) return -2;
   if (vec) {
-    GB_DISPATCH_FLOAT(dt, T, moe_combine_bwd_vec_kernel<T><<<gb_grid(tokens * k * 32, 256), 256, 0, st>>>(
-        (const T*)g, (const T*)y, w, pos, (T*)dy, dw, tokens, k, cols));
-    return (int)cudaGetLastError();
+    const long long units = row_token != nullptr && rows > tokens * k ? rows : tokens * k;
+    if (units == 0) return 0;
+    const int nv = (int)((long long)cols * es / 16);
+    auto launch = [&](auto lpr) {
+      constexpr int L = decltype(lpr)::value;
+      GB_DISPATCH_FLOAT(dt, T, moe_combine_bwd_vec_kernel<T, L><<<gb_grid(units * L, 256), 256, 0, st>>>(
+          (const T*)g, (const T*)y, w, pos, row_token, (T*)dy, dw, tokens, rows, k, cols));
+      return (int)cudaGetLastError();
+    };
+    if (nv <= 8) return launch(std::integral_constant<int, 8>{});
+    if (nv <= 16) return launch(std::integral_constant<int, 16>{});
+    return launch(std::integral_constant<int, 32>{});
   }
+  if (tokens == 0) return 0;
   GB_DISPATCH_FLOAT(dt, T, moe_combine_bwd_kernel<T><<<gb_grid(tokens * k * 32, 256), 256, 0, st>>>(
       (const T*)g, (const T*)y, w, pos, (T*)dy, dw, tokens, k, cols));
   return (int)cudaGetLastError();

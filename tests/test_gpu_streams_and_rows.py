@@ -69,7 +69,8 @@ def test_cross_entropy_rows(cols, dt):
     assert float(loss[4]) == 0.0
 
 
-@pytest.mark.parametrize("T,k,E,cols", [(1, 1, 2, 8), (37, 2, 8, 136), (300, 8, 16, 2048), (129, 8, 128, 256), (64, 3, 5, 20)])
+@pytest.mark.parametrize("T,k,E,cols", [(1, 1, 2, 8), (37, 2, 8, 136), (300, 8, 16, 2048), (129, 8, 128, 256), (64, 3, 5, 20),
+                                        (50, 4, 8, 64), (50, 4, 8, 72), (77, 2, 8, 128)])
 def test_moe_row_sums(T, k, E, cols):
     g = torch.Generator(device=DEV).manual_seed(T)
     e = torch.rand(T, E, device=DEV, generator=g).topk(k, 1).indices.int().contiguous()
