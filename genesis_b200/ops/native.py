@@ -90,9 +90,16 @@ def lib():
 available = _lib.available
 
 
+# read on every launch, so without the Stream object around the handle; the names are torch's own, hence the other way
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_this_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _st():
-    # the raw handle of the current device's current stream, without the Stream object around it: read on every launch
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    """Raw handle of the current device's current stream."""
+    if _raw_stream is None or _this_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_this_device())
 
 
 launch_count = 0   # native launches since import (every wrapper call below launches >= 1 kernel)

@@ -106,3 +106,15 @@ def test_kernels_that_give_up_wait_for_their_copies():
         # a barrier is always past one of its two parities, so a wait for either of them ends at once
         assert not re.search(r"!mbar_try_wait\(&?([^,]+), 0\) && !mbar_try_wait\(&?\1, 1\)", body), (f, name)
     assert seen >= 9
+
+
+@pytest.mark.parametrize("gone", ["_raw_stream", "_this_device"])
+def test_stream_handle_without_torchs_private_names(monkeypatch, gone):
+    class Stream:
+        cuda_stream = 7
+    monkeypatch.setattr(N, "_raw_stream", lambda device: 100 + device)
+    monkeypatch.setattr(N, "_this_device", lambda: 3)
+    assert N._st() == 103
+    monkeypatch.setattr(N, gone, None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: Stream)
+    assert N._st() == 7
