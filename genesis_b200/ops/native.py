@@ -90,16 +90,15 @@ def lib():
 available = _lib.available
 
 
-# read on every launch, so without the Stream object around the handle; the names are torch's own, hence the other way
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_this_device = getattr(torch._C, "_cuda_getDevice", None)
+def _stream_handle(raw, device):
+    """Function that returns the raw handle of the current device's current stream.  It is called on every launch, so it
+    does without the Stream object around the handle where torch has its (private) names for that."""
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
 
 
-def _st():
-    """Raw handle of the current device's current stream."""
-    if _raw_stream is None or _this_device is None:
-        return torch.cuda.current_stream().cuda_stream
-    return _raw_stream(_this_device())
+_st = _stream_handle(getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None))
 
 
 launch_count = 0   # native launches since import (every wrapper call below launches >= 1 kernel)
@@ -326,25 +325,31 @@ def cast(t, dtype):
     return out
 
 
+_LONGS = [ctypes.c_longlong * i for i in range(9)]
+
+
 def cast_stack(tensors, out):
     """Up to eight fp32 tensors converted into the 16-bit `out`, one after another along dim 0, by one launch.  All have
     to lie on the device of `out`, and their rows have to be those of `out`: the caller's copies, one by one, take (or
     refuse) anything else."""
     n = len(tensors)
-    if n > 8 or out.dtype not in (torch.bfloat16, torch.float16) or not out.is_contiguous() or out.data_ptr() % 16:
+    dt = out.dtype
+    if n > 8 or (dt is not BF16 and dt is not F16) or not out.is_contiguous() or out.data_ptr() % 16:
         return NotImplemented
-    src, num = [], []
-    dev, row = out.device, out.shape[1:]
+    src, num = _LONGS[n](), _LONGS[n]()
+    dev, row = out.get_device(), out.stride()        # (contiguous tensors: the strides are those of the trailing dims)
+    left, i = out.numel(), 0
     for t in tensors:
         p, k = t.data_ptr(), t.numel()
-        if t.dtype != F32 or t.device != dev or t.shape[1:] != row or not t.is_contiguous() or p % 16 or k % 8 or k == 0:
+        if t.dtype is not F32 or t.get_device() != dev or t.stride() != row or not t.is_contiguous() or p % 16 or k % 8 \
+                or k == 0:
             return NotImplemented
-        src.append(p)
-        num.append(k)
-    if sum(num) != out.numel():
+        src[i], num[i] = p, k
+        left -= k
+        i += 1
+    if left:
         return NotImplemented
-    _chk(lib().gb_cast_stack((ctypes.c_longlong * n)(*src), (ctypes.c_longlong * n)(*num), n, out.data_ptr(),
-                             _DT[out.dtype], _st()), "cast_stack")
+    _chk(lib().gb_cast_stack(src, num, n, out.data_ptr(), _DT[dt], _st()), "cast_stack")
     return out
 
 
@@ -875,7 +880,7 @@ def _norm_ok(x, cols):
 
 def _weights_ok(x, w, cols):
     """Weights (or biases) that the row kernels can read in 16-byte pieces: one per column, on the device of x."""
-    return w.numel() == cols and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.device == x.device
+    return w.numel() == cols and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.get_device() == x.get_device()
 
 
 def _wdt(x, w):
@@ -1134,16 +1139,17 @@ def _token_rows(t):
     return rs, True
 
 
-def _tables_ok(dev, cos, sin, positions):
-    """Rotation tables (and positions) that a kernel on `dev` can read: one left on the host, by a module that was not
-    moved, is torch's to take or to refuse."""
-    return (cos.dtype == F32 and sin.dtype == F32 and cos.device == dev and sin.device == dev and cos.is_contiguous()
-            and sin.is_contiguous() and (positions is None or positions.device == dev))
+def _tables_ok(x, cos, sin, positions):
+    """Rotation tables (and positions) that a kernel on the device of `x` can read: one left on the host, by a module that
+    was not moved, is torch's to take or to refuse."""
+    dev = x.get_device()
+    return (cos.dtype == F32 and sin.dtype == F32 and cos.get_device() == dev and sin.get_device() == dev
+            and cos.is_contiguous() and sin.is_contiguous() and (positions is None or positions.get_device() == dev))
 
 
 def rope(x, cos, sin, positions, inverse, out=None):
     """Rotate-half RoPE.  `x` and `out` may be column slices of wider matrices (equal token-row spacing)."""
-    if x.dtype not in _FLOATS or x.dim() != 4 or x.shape[-1] % 2 or not _tables_ok(x.device, cos, sin, positions):
+    if x.dtype not in _FLOATS or x.dim() != 4 or x.shape[-1] % 2 or not _tables_ok(x, cos, sin, positions):
         return NotImplemented
     xrs, ok = _token_rows(x)
     if not ok:
@@ -1172,7 +1178,7 @@ def qkv_rope(y, q, k, v, cos, sin, positions, Hq, Hkv, D, merge):
     rotated q, rotated k, v, all freshly allocated when passed as None) or merge (`merge=True`: gradients q, k, v ->
     y, rotated back).  Returns (y, q, k, v) or NotImplemented."""
     t = y if y is not None else q
-    if t.dtype not in _FLOATS or not _tables_ok(t.device, cos, sin, positions):
+    if t.dtype not in _FLOATS or not _tables_ok(t, cos, sin, positions):
         return NotImplemented
     B, S = t.shape[0], t.shape[1]
     Nt = (Hq + 2 * Hkv) * D

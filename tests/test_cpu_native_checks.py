@@ -11,6 +11,16 @@ from genesis_b200.ops import dispatch as K
 from genesis_b200.ops import native as N
 
 
+class _Elsewhere(torch.Tensor):
+    """A tensor of another device, as far as the wrappers look."""
+    def get_device(self):
+        return 5
+
+
+def _elsewhere(t):
+    return t.as_subclass(_Elsewhere)
+
+
 class _Recorder:
     def __init__(self):
         self.calls = []
@@ -36,7 +46,7 @@ def test_stacked_conversion_takes_one_device_and_whole_rows(native):
     out = torch.empty(6, 8, dtype=torch.bfloat16)
     assert N.cast_stack([a, b], out) is out and native.calls == ["gb_cast_stack"]
     native.calls.clear()
-    for ts in ([a, b.to("meta")], [a.to("meta"), b], [a, torch.randn(4, 4)], [a, torch.randn(16)], [a, torch.randn(1, 8)]):
+    for ts in ([a, _elsewhere(b)], [_elsewhere(a), b], [a, torch.randn(4, 4)], [a, torch.randn(16)], [a, torch.randn(1, 8)]):
         assert N.cast_stack(ts, out) is NotImplemented
     assert native.calls == []
     # rows that do not match are refused by the copies, as a concatenation would
@@ -58,7 +68,7 @@ def test_rotation_tables_of_another_device(native, away):
         return [x is NotImplemented for x in r], len(native.calls)
 
     assert launches() == ([False] * 3, 3)
-    t[away] = t[away].to("meta")
+    t[away] = _elsewhere(t[away])
     assert launches() == ([True] * 3, 0)
 
 
@@ -80,7 +90,7 @@ def test_norm_weights_that_the_kernels_cannot_read(native, monkeypatch, wdt):
     base = torch.ones(2 * cols + 8, dtype=wdt)
     assert base.data_ptr() % 16 == 0
     assert refused(base[:cols]) == ({False}, 7)
-    for w in (base[1:cols + 1], base[:2 * cols:2], base[:cols].to("meta"), base[:cols - 1], base[:1]):
+    for w in (base[1:cols + 1], base[:2 * cols:2], _elsewhere(base[:cols]), base[:cols - 1], base[:1]):
         assert refused(w) == ({True}, 0)
 
 
@@ -108,13 +118,10 @@ def test_kernels_that_give_up_wait_for_their_copies():
     assert seen >= 9
 
 
-@pytest.mark.parametrize("gone", ["_raw_stream", "_this_device"])
-def test_stream_handle_without_torchs_private_names(monkeypatch, gone):
+def test_stream_handle_without_torchs_private_names(monkeypatch):
     class Stream:
         cuda_stream = 7
-    monkeypatch.setattr(N, "_raw_stream", lambda device: 100 + device)
-    monkeypatch.setattr(N, "_this_device", lambda: 3)
-    assert N._st() == 103
-    monkeypatch.setattr(N, gone, None)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda: Stream)
-    assert N._st() == 7
+    raw, device = (lambda d: 100 + d), (lambda: 3)
+    assert N._stream_handle(raw, device)() == 103
+    assert N._stream_handle(None, device)() == 7 and N._stream_handle(raw, None)() == 7
