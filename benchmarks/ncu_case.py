@@ -6,8 +6,9 @@
 
 Cases (kernel to pass to -k): gemm_pair, gemm_swiglu, gemm_swiglu_bwd (gemm2_kernel), gemm (gemm_kernel),
 grouped_gemm (gemm_kernel), attn128_fwd (attn_fwd_kernel), attn128_bwd (attn_bwd_dq_kernel / attn_bwd_dkdv_kernel),
-attn64_fwd, attn64_bwd, ce (ce_fwd_kernel / ce_bwd_kernel), softmax (row_stream_kernel / softmax_bwd), rmsnorm (row_stream_kernel / rmsnorm_bwd_kernel),
-addnorm, adam (adam_multi_kernel), swiglu_bwd (swiglu_bwd2d_kernel), rope (rope_vec_kernel),
+attn64_fwd, attn64_bwd, attn_decode (attn_decode_kernel), ce (ce_fwd16_kernel / ce_bwd_kernel), softmax (row_stream_kernel / softmax_bwd), rmsnorm (row_stream_kernel / rmsnorm_bwd_kernel),
+addnorm, addnorm_wide (add_rmsnorm_fwd_stream_kernel / rmsnorm_bwd_stream_kernel), moe_combine_bwd (moe_combine_bwd_vec_kernel),
+adam (adam_multi_kernel), swiglu_bwd (swiglu_bwd2d_kernel), rope (rope_vec_kernel),
 reduce_cols (reduce_mid), sort (sort_rows), index (index_get_kernel / index_put_kernel), cat (cat_kernel).
 """
 import sys
@@ -69,6 +70,11 @@ def _attn(B, S, Hq, Hkv, D, bwd):
     return lambda: K.attention_bwd(do, q, k, v, o, lse, True, scale)
 
 
+def attn_decode():
+    q, k, v = rnd(64, 1, 32, 128), rnd(64, 4096, 4, 128), rnd(64, 4096, 4, 128)
+    return lambda: K.attention_fwd(q, k, v, True, 128 ** -0.5)
+
+
 def ce():
     logits = rnd(4096, 151936)
     tgt = torch.randint(0, 151936, (4096,), device=DEV)
@@ -97,13 +103,20 @@ def rmsnorm():
     return f
 
 
-def addnorm():
-    x, r, w, g = rnd(65536, 896), rnd(65536, 896), torch.ones(896, device=DEV), rnd(65536, 896)
+def addnorm(rows=65536, cols=896):
+    x, r, w, g = rnd(rows, cols), rnd(rows, cols), torch.ones(cols, device=DEV), rnd(rows, cols)
 
     def f():
         s, y, rstd = K.add_rmsnorm_fwd(x, r, w, 1e-6)
         K.add_rmsnorm_bwd(g, g, s, w, rstd)
     return f
+
+
+def moe_combine_bwd():
+    e = torch.rand(16384, 64, device=DEV).topk(8, 1).indices.int().contiguous()
+    token_of, pos, _ = K.moe_sort(e, 64)
+    y, g, w = rnd(token_of.numel(), 2048), rnd(16384, 2048), torch.rand(16384, 8, device=DEV)
+    return lambda: K.moe_combine_bwd(g, y, w, pos, token_of)
 
 
 def adam():
@@ -157,6 +170,7 @@ CASES = {
     "gemm_pair": gemm_pair, "gemm_swiglu": gemm_swiglu, "gemm_swiglu_bwd": gemm_swiglu_bwd, "gemm": gemm, "grouped_gemm": grouped_gemm,
     "attn128_fwd": lambda: _attn(4, 4096, 16, 4, 128, False), "attn128_bwd": lambda: _attn(4, 4096, 16, 4, 128, True),
     "attn64_fwd": lambda: _attn(8, 2048, 14, 2, 64, False), "attn64_bwd": lambda: _attn(8, 2048, 14, 2, 64, True),
+    "attn_decode": attn_decode, "addnorm_wide": lambda: addnorm(8192, 4096), "moe_combine_bwd": moe_combine_bwd,
     "ce": ce, "softmax": softmax, "rmsnorm": rmsnorm, "addnorm": addnorm, "adam": adam, "swiglu_bwd": swiglu_bwd,
     "rope": rope, "reduce_cols": reduce_cols, "sort": sort, "index": index, "cat": cat,
 }
