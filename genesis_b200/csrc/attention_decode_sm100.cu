@@ -4,8 +4,10 @@
 // query rows of all heads of a KV head's group (S * Hq / Hkv of them) are the rows of one 16-row tile, K and V are read
 // once per 16 such rows, and the keys are split between the CTAs of a cluster, which combine their partial results
 // through distributed shared memory: one launch, no workspace.
-//   measured : 8 x 1 queries, 32 / 4 heads of 128, 4096 keys: 107 us with 128-row tiles, 19 us here (3.4 TB/s of K and V);
-//              1 x 1, 14 / 2 heads of 64, 8192 keys: 101 -> 12.5 us.  Launch and cluster barriers take about 8 us of each.
+//   measured : time on the GPU, inputs cycled past L2: 8 x 1 queries, 32 / 4 heads of 128, 4096 keys: 112 us with 128-row
+//              tiles, 18.9 us here (3.6 TB/s of K and V; 64 x 1, 4096 keys: 90 us, 6.0 TB/s); 1 x 1, 14 / 2 heads of 64, 8192
+//              keys: 101 -> 12 us.  Launch, ring start and cluster barriers are about 6 us of each: 64 keys take 6.2.  Against the
+//              tiled kernel by shape: decode_wins in attention_sm100.cu.
 //   bound    : the bytes of K and V.  Every warp streams its own chunks of keys through a private three-stage TMA ring (no
 //              barrier between warps in the loop) and multiplies them with mma.sync: with 16 rows the arithmetic is far
 //              below what the loads take, and a 128-row tcgen05 tile would be mostly padding.

@@ -10,8 +10,11 @@
 // probabilities go back as 16-bit pairs into the columns of the score tile they came from: P is the tensor-memory A
 // operand of the second GEMM and shared memory holds only what TMA wrote (Q tiles, a ring of K / V tiles) and the
 // per-warp slabs of the output store.
-//   bound       : the exponentials (one MUFU result per score, 16 per clock and SM: 1024 clocks a tile) at D = 64, which
-//                 is twice the tensor time there; at D = 128 the two come to the same 1024 clocks.
+//   bound       : per tile and SM the exponentials take 1024 clocks (one MUFU result per score, 16 per clock), the products
+//                 512 at D = 64 and 1024 at D = 128.  At D = 64 a quarter of the exponentials of a tile without a mask goes to
+//                 the FMA pipes, which leaves 768 clocks of MUFU beside the FMA work.
+//   registers   : ten warps put three on one scheduler, which caps every warp at 168 registers; the soft-max loop spills 44
+//                 bytes at D = 128 and 32 at D = 64.
 //   rescaling   : the accumulator is multiplied only when a row maximum grows by more than 2^8 over the reference it was
 //                 started with; probabilities up to 2^8 keep their relative precision in 16 and 32 bits, and the final
 //                 division by the row sum (taken against the same reference) removes the factor.
