@@ -50,7 +50,7 @@ def test_wide_rmsnorm(rows, cols, dt):
         assert torch.equal(dx, again[0]) and torch.equal(dw, again[1])
 
 
-@pytest.mark.parametrize("cols", [8, 1000, 4096, 4096 + 8, 8192 - 8, 32771, 65536 - 8, 65536, 65536 + 3, 151936])
+@pytest.mark.parametrize("cols", [8, 1000, 4096, 5120 - 8, 5120, 5121, 8192 - 8, 32771, 65536 - 8, 65536, 65536 + 3, 151936])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
 def test_cross_entropy_rows(cols, dt):
     x = _rnd(6, cols, dt=dt) * 4
